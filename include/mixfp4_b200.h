@@ -177,6 +177,19 @@ MIXFP4_API int mixfp4_e0_four_over_six(const float* grouped, int64_t nblocks, co
                             float* codes, float* dequant, float* scales, float* errors,
                             uint8_t* expansion_ids, void* stream);
 
+/* mixfp4_fake_quantize with one format per region of region_rows x region_groups K16 blocks (the regions
+ * mixfp4_select_regions knows whose row counts are powers of two up to 64; same sums, same decisions) in one amax
+ * and one quantizer pass.  amax: device float scratch.  y must not alias x. */
+MIXFP4_API int mixfp4_fake_quantize_regions(const void* x, int dtype, int64_t rows, int64_t k, int64_t ldx,
+                                 int region_rows, int region_groups, float* amax, void* y, int64_t ldy,
+                                 void* stream);
+
+/* mixfp4_quantize (modes oracle16, all_e2m1, all_e0m3) writing the stream layout directly: chunks has
+ * mixfp4_stream_bytes(rows, k) bytes and receives what mixfp4_repack_stream makes of mixfp4_quantize's outputs.
+ * lut (optional): 36864 bytes, receives mixfp4_decode_table_wide's table. */
+MIXFP4_API int mixfp4_quantize_stream(const void* x, int dtype, int64_t rows, int64_t k, int64_t ldx, int mode,
+                           const float* amax, uint8_t* chunks, float* global_scale, void* lut, void* stream);
+
 /* Packed -> dense weight in out_dtype (the tensor the reference stores back into
  * nn.Linear.weight, project_quant/modeling.py:629). */
 MIXFP4_API int mixfp4_dequant(const uint8_t* codes, const uint8_t* scales, const uint8_t* fmt,
@@ -219,6 +232,11 @@ MIXFP4_API int mixfp4_decode_table_wide(const float* global_scale, void* lut, vo
  * stages and rounds once at the end. */
 MIXFP4_API int mixfp4_fwht(const void* x, void* y, int dtype, int64_t rows, int64_t k, int64_t ldx,
                 int64_t ldy, int size, const float* signs, int stagewise, void* stream);
+
+/* mixfp4_fwht followed by mixfp4_amax of its result (*amax: device float), in one pass where the rows are
+ * whole aligned H128 blocks of a 16-bit type, rounded stage by stage, without signs. */
+MIXFP4_API int mixfp4_fwht_amax(const void* x, void* y, int dtype, int64_t rows, int64_t k, int64_t ldx,
+                     int64_t ldy, int size, const float* signs, int stagewise, float* amax, void* stream);
 
 /* Decode-shape dequant-linear, 1 <= M <= 16: y[M,N] = x[M,K] * W[N,K]^T with W packed
  * (replaces F.linear on the dequantized weight, modeling.py:629 + nn.Linear.forward).

@@ -69,6 +69,10 @@ def _declare(h: ctypes.CDLL) -> None:
     h.mixfp4_quantize.argtypes = [p, i32, i64, i64, i64, i32, p, p, p, p, p, p, p, p, p, p, i64, p]
     h.mixfp4_fake_quantize.restype = i32
     h.mixfp4_fake_quantize.argtypes = [p, i32, i64, i64, i64, i32, p, p, i64, p]
+    h.mixfp4_fake_quantize_regions.restype = i32
+    h.mixfp4_fake_quantize_regions.argtypes = [p, i32, i64, i64, i64, i32, i32, p, p, i64, p]
+    h.mixfp4_quantize_stream.restype = i32
+    h.mixfp4_quantize_stream.argtypes = [p, i32, i64, i64, i64, i32, p, p, p, p, p]
     h.mixfp4_select_regions.restype = i32
     h.mixfp4_select_regions.argtypes = [p, p, i64, i64, i32, i32, p, p]
     h.mixfp4_select_layer.restype = i32
@@ -89,6 +93,8 @@ def _declare(h: ctypes.CDLL) -> None:
     h.mixfp4_decode_table.argtypes = [p, p, p]
     h.mixfp4_fwht.restype = i32
     h.mixfp4_fwht.argtypes = [p, p, i32, i64, i64, i64, i64, i32, p, i32, p]
+    h.mixfp4_fwht_amax.restype = i32
+    h.mixfp4_fwht_amax.argtypes = [p, p, i32, i64, i64, i64, i64, i32, p, i32, p, p]
     h.mixfp4_gemv.restype = i32
     h.mixfp4_gemv.argtypes = [p, i64, i64, p, p, p, p, i64, i64, i32, p, p, i32, i64, i32, p]
     h.mixfp4_gemv_grouped.restype = i32
@@ -138,7 +144,7 @@ def _declare(h: ctypes.CDLL) -> None:
 # every symbol include/mixfp4_b200.h declares
 EXPORTED = (
     "mixfp4_abi_version", "mixfp4_status_string", "mixfp4_last_cuda_error", "mixfp4_padded_k",
-    "mixfp4_amax", "mixfp4_quantize", "mixfp4_fake_quantize", "mixfp4_select_regions", "mixfp4_select_layer", "mixfp4_selftest_division", "mixfp4_round_codebook", "mixfp4_e0_four_over_six", "mixfp4_dequant", "mixfp4_repack", "mixfp4_decode_table", "mixfp4_decode_table_wide", "mixfp4_fwht",
+    "mixfp4_amax", "mixfp4_quantize", "mixfp4_fake_quantize", "mixfp4_fake_quantize_regions", "mixfp4_quantize_stream", "mixfp4_select_regions", "mixfp4_select_layer", "mixfp4_selftest_division", "mixfp4_round_codebook", "mixfp4_e0_four_over_six", "mixfp4_dequant", "mixfp4_repack", "mixfp4_decode_table", "mixfp4_decode_table_wide", "mixfp4_fwht", "mixfp4_fwht_amax",
     "mixfp4_stream_bytes", "mixfp4_repack_stream", "mixfp4_repack_from_stream",
     "mixfp4_gemv", "mixfp4_gemv_x_fits", "mixfp4_gemv_grouped",
     "mixfp4_comm_create", "mixfp4_comm_handle_bytes", "mixfp4_comm_handle", "mixfp4_comm_open",

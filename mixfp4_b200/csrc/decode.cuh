@@ -58,16 +58,12 @@ __device__ __forceinline__ void decode8(uint32_t w, const uint4& t, uint32_t (&p
 //           and one shift+mask (elements 4..7) put the signs on bit 7 of the high bytes;
 //   scales: bit 7 of the E4M3 byte (always 0 for a block scale) carries the block's format
 //           bit, so the byte is the table index and no format array is read.
-__host__ __device__ __forceinline__ uint32_t codes_to_kernel_layout(uint32_t w) {
-    uint32_t out = w & 0x77777777u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        out |= ((w >> (4 * i + 3)) & 1u) << (8 * i + 7);          // sign of element i
-        out |= ((w >> (4 * (4 + i) + 3)) & 1u) << (8 * i + 3);    // sign of element 4 + i
-    }
-    return out;
+__device__ __forceinline__ uint32_t codes_to_kernel_layout(uint32_t w) {
+    const uint32_t w4 = w << 4;                       // the signs of even elements on bit 7 of their bytes
+    const uint32_t a = prmt(w, w4, 0x1504u) & 0x80808080u, b = prmt(w, w4, 0x3726u) & 0x80808080u;   // elements 0..3, 4..7
+    return (w & 0x77777777u) | a | (b >> 4);
 }
-__host__ __device__ __forceinline__ uint32_t codes_from_kernel_layout(uint32_t w) {
+__device__ __forceinline__ uint32_t codes_from_kernel_layout(uint32_t w) {
     uint32_t out = w & 0x77777777u;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {

@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kFastThreads) fwht128_stagewise_kernel(const T
                                                                          unsigned int* __restrict__ amax) {
     using P = Pair<T>;
     using T2 = typename P::type;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the quantizer behind it, see fwht128_kernel
     const int lane = threadIdx.x & 31, h = lane & 1;
     const int64_t warp = (int64_t)blockIdx.x * (kFastThreads / 32) + (threadIdx.x >> 5);
     const int64_t blk = warp * kFastBlocksPerWarp + (lane >> 1);
@@ -477,4 +478,16 @@ extern "C" int mixfp4_fwht(const void* x, void* y, int dtype, int64_t rows, int6
         case MIXFP4_F32: return launch<float>(x, y, rows, k, ldx, ldy, size, signs, stagewise, st);
         default: return MIXFP4_E_DTYPE;
     }
+}
+
+extern "C" int mixfp4_fwht_amax(const void* x, void* y, int dtype, int64_t rows, int64_t k, int64_t ldx, int64_t ldy,
+                                int size, const float* signs, int stagewise, float* amax, void* stream) {
+    if (!x || !y || !amax) return MIXFP4_E_NULL;
+    if (rows <= 0 || k <= 0 || ldx < k || ldy < k) return MIXFP4_E_SHAPE;
+    if (size == 128 && !signs && stagewise) {
+        const int rc = fwht128_stagewise_amax(x, y, dtype, rows, k, ldx, ldy, amax, static_cast<cudaStream_t>(stream));
+        if (rc != MIXFP4_E_UNSUPPORTED) return rc;
+    }
+    if (const int rc = mixfp4_fwht(x, y, dtype, rows, k, ldx, ldy, size, signs, stagewise, stream)) return rc;
+    return mixfp4_amax(y, dtype, rows, k, ldy, amax, stream);
 }

@@ -33,6 +33,8 @@ constexpr int kWarpsPerCta = kThreads / 32;
 template <typename T>
 __global__ void __launch_bounds__(kThreads) amax_kernel(const T* __restrict__ x, int64_t rows, int64_t k,
                                                         int64_t ldx, bool vec, unsigned int* __restrict__ out) {
+    // the quantizer behind this kernel may set itself up while this grid runs (it waits for the grid's end)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     float m = 0.0f;
     if (vec) {
         // rows are contiguous 16-byte multiples: walk the tensor as uint4 words
@@ -118,11 +120,6 @@ __device__ __forceinline__ float div_rcp(float a, float b, float r) {
     const float rem = __fmaf_rn(-q, b, a);
     return __fmaf_rn(rem, r, q);
 }
-template <bool kFast>
-__device__ __forceinline__ float div_exact(float a, float b, float r) {
-    if constexpr (kFast) return div_rcp(a, b, r);
-    else return __fdiv_rn(a, b);
-}
 
 // E2M1 rounding of |n| exactly as codebook.py:12-25 computes it: exponent floor(log2 |n|)
 // clamped at 0, floor(mantissa * 2 + 0.5), saturate at 6.  For |n| >= 1 that is round-half-up
@@ -172,22 +169,21 @@ __device__ __forceinline__ float2 e2m1_pair_levels(uint32_t byte) {
 // One candidate format of one block.  ax = |x|, s = x / gs.  Produces the block's scale, its
 // squared error in the reference's summation order, the magnitudes of the dequantized values
 // (kKeep) and the eight-per-word 3-bit level codes without signs (kPack).
-template <bool kE0, bool kFast, bool kPack, bool kKeep>
+template <bool kE0, bool kPack, bool kKeep>
 __device__ __forceinline__ void candidate(const float (&ax)[kGroup], const float (&s)[kGroup], float amax_s,
                                           float gs, uint32_t& lo, uint32_t& hi, uint32_t& scale_byte,
                                           float& scale_val, float& err, float (&dmag)[kGroup]) {
-    float ideal = div_exact<kFast>(amax_s, kE0 ? 7.0f : 6.0f, kE0 ? (1.0f / 7.0f) : (1.0f / 6.0f));
+    float ideal = __fdiv_rn(amax_s, kE0 ? 7.0f : 6.0f);
     ideal = fminf(fmaxf(ideal, 0.001953125f), 448.0f);
     scale_byte = __nv_cvt_float_to_fp8(ideal, __NV_SATFINITE, __NV_E4M3);
     const float sc = e4m3_to_float(scale_byte);
-    const float rsc = __frcp_rn(sc);
     scale_val = sc;
     float sq[kGroup];
     float p4[4] = {0.0f, 0.0f, 0.0f, 0.0f};         // E0M3: four levels per float, 16^j weights (exact)
     uint32_t byte[8];                               // E2M1: code bytes of the eight element pairs
 #pragma unroll
     for (int i = 0; i < kGroup; i += 2) {
-        const float mag0 = fabsf(div_exact<kFast>(s[i], sc, rsc)), mag1 = fabsf(div_exact<kFast>(s[i + 1], sc, rsc));
+        const float mag0 = fabsf(__fdiv_rn(s[i], sc)), mag1 = fabsf(__fdiv_rn(s[i + 1], sc));
         float q[2];
         if constexpr (kE0) {
             q[0] = e0m3_round(mag0);
@@ -245,6 +241,15 @@ __device__ __forceinline__ float2 div_rcp2(float2 a, float2 neg_b, float2 r) {
     const float2 rem = __ffma2_rn(q, neg_b, a);
     return __ffma2_rn(rem, r, q);
 }
+// The same with one more correction, for dividends with a full fp32 significand and any divisor whose
+// significand is not all ones: the first correction makes q faithful (within one unit in the last place), and
+// Markstein's theorem (P. W. Markstein, IBM J. Res. Dev. 34, 1990) says that correcting a faithful q once more
+// with the correctly rounded reciprocal gives the IEEE quotient.  The quotient of -0 is +0 as above.
+__device__ __forceinline__ float2 div_rcp2_twice(float2 a, float2 neg_b, float2 r) {
+    const float2 q = div_rcp2(a, neg_b, r);
+    const float2 rem = __ffma2_rn(q, neg_b, a);
+    return __ffma2_rn(rem, r, q);
+}
 // The nudge of e2m1_nudge for a signed pair, without a comparison.  Adding 2^-27 with the value's sign first:
 // at 0.25 and above that is at most a quarter of the spacing and rounds back to the value; between 0.125 and
 // 0.25 it is half the spacing, so values with an odd last bit move up one step -- all of them stay below 0.25
@@ -277,24 +282,31 @@ __device__ __forceinline__ float error_sum(const float2 (&sq)[8]) {
     }
     return acc;
 }
-// x2[j] = elements (2j, 2j+1) of the block.  d2 / d0: signed dequantized values (kKeep).
+// Both candidates of one block.  e2: E2M1, e0: E0M3.
 template <bool kPack, bool kKeep>
-__device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs, float rgs, uint32_t& lo2, uint32_t& hi2,
-                                                uint32_t& b2, float& sc2, float& err2, float2 (&d2)[8], uint32_t& lo0,
-                                                uint32_t& hi0, uint32_t& b0, float& sc0, float& err0, float2 (&d0)[8]) {
+struct BlockCandidates {
+    uint32_t lo2, hi2, lo0, hi0;     // kPack: level codes of elements 0..7 / 8..15 (E2M1 words with their sign bits)
+    uint32_t byte2, byte0;           // E4M3 scale bytes
+    float sc2, sc0, err2, err0;
+    float2 d2[8], d0[8];             // kKeep: dequantized values; d2 has the sign of x, a zero of d0 may lack it
+};
+
+// x2[j] = elements (2j, 2j+1) of the block; the packed path.  kWide: x has a full fp32 significand.
+template <bool kWide, bool kPack, bool kKeep>
+__device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs, float rgs, BlockCandidates<kPack, kKeep>& o) {
     const float2 rgs2 = make_float2(rgs, rgs), ngs2 = make_float2(-gs, -gs), gs2 = make_float2(gs, gs);
     const float2 neg1 = make_float2(-1.0f, -1.0f);
     float2 s[8];
     float amax_s = 0.0f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        s[j] = div_rcp2(x2[j], ngs2, rgs2);
+        s[j] = kWide ? div_rcp2_twice(x2[j], ngs2, rgs2) : div_rcp2(x2[j], ngs2, rgs2);
         amax_s = fmaxf(amax_s, fmaxf(fabsf(s[j].x), fabsf(s[j].y)));      // |.| folds into the (three-input) maximum
     }
     {   // E2M1
         float rsc;
-        block_scale_fast<false>(amax_s, b2, sc2, rsc);
-        const float2 rsc2 = make_float2(rsc, rsc), nsc2 = make_float2(-sc2, -sc2), scv = make_float2(sc2, sc2);
+        block_scale_fast<false>(amax_s, o.byte2, o.sc2, rsc);
+        const float2 rsc2 = make_float2(rsc, rsc), nsc2 = make_float2(-o.sc2, -o.sc2), scv = make_float2(o.sc2, o.sc2);
         float2 sq[8];
         uint32_t byte[8];
 #pragma unroll
@@ -302,43 +314,172 @@ __device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs,
             const float2 n = div_rcp2(s[j], nsc2, rsc2);
             byte[j] = __nv_cvt_float2_to_fp4x2(e2m1_nudge_pair(n), __NV_E2M1, cudaRoundNearest);
             const float2 d = __fmul2_rn(__fmul2_rn(e2m1_pair_levels(byte[j]), scv), gs2);
-            if constexpr (kKeep) d2[j] = d;
+            if constexpr (kKeep) o.d2[j] = d;
             const float2 e = __ffma2_rn(x2[j], neg1, d);
             sq[j] = __fmul2_rn(e, e);
         }
-        err2 = error_sum(sq);
-        lo2 = hi2 = 0;
+        o.err2 = error_sum(sq);
         if constexpr (kPack) {
-            lo2 = __byte_perm(__byte_perm(byte[0], byte[1], 0x0040), __byte_perm(byte[2], byte[3], 0x0040), 0x5410);
-            hi2 = __byte_perm(__byte_perm(byte[4], byte[5], 0x0040), __byte_perm(byte[6], byte[7], 0x0040), 0x5410);
+            o.lo2 = __byte_perm(__byte_perm(byte[0], byte[1], 0x0040), __byte_perm(byte[2], byte[3], 0x0040), 0x5410);
+            o.hi2 = __byte_perm(__byte_perm(byte[4], byte[5], 0x0040), __byte_perm(byte[6], byte[7], 0x0040), 0x5410);
         }
     }
     {   // E0M3
         float rsc;
-        block_scale_fast<true>(amax_s, b0, sc0, rsc);
-        const float2 rsc2 = make_float2(rsc, rsc), nsc2 = make_float2(-sc0, -sc0), scv = make_float2(sc0, sc0);
+        block_scale_fast<true>(amax_s, o.byte0, o.sc0, rsc);
+        const float2 rsc2 = make_float2(rsc, rsc), nsc2 = make_float2(-o.sc0, -o.sc0), scv = make_float2(o.sc0, o.sc0);
         const float2 magic = make_float2(12582912.0f, 12582912.0f), nmagic = make_float2(-12582912.0f, -12582912.0f);
-        float2 sq[8];
+        float2 n[8], sq[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) n[j] = div_rcp2(s[j], nsc2, rsc2);
+        // Levels above 7 only occur where the scale was rounded down by more than 1/15 (7.49 = 7 * 1.07), which
+        // a scale with its four significand bits never is: the clamp is a rare branch.
+        if (amax_s > __fmul_rn(7.49f, o.sc0)) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                n[j] = make_float2(fminf(fmaxf(n[j].x, -7.25f), 7.25f), fminf(fmaxf(n[j].y, -7.25f), 7.25f));
+        }
         float p4[4] = {0.0f, 0.0f, 0.0f, 0.0f};         // four levels per float, 16^j weights (exact)
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const float2 n = div_rcp2(s[j], nsc2, rsc2);
-            const float2 c = make_float2(fminf(fmaxf(n.x, -7.25f), 7.25f), fminf(fmaxf(n.y, -7.25f), 7.25f));
-            const float2 q = __fadd2_rn(__fadd2_rn(c, magic), nmagic);
+            const float2 q = __fadd2_rn(__fadd2_rn(n[j], magic), nmagic);
             if constexpr (kPack)
                 p4[j >> 1] = (j & 1) == 0 ? __fmaf_rn(fabsf(q.y), 16.0f, fabsf(q.x))
                                           : __fmaf_rn(fabsf(q.y), 4096.0f, __fmaf_rn(fabsf(q.x), 256.0f, p4[j >> 1]));
             const float2 d = __fmul2_rn(__fmul2_rn(q, scv), gs2);
-            if constexpr (kKeep) d0[j] = d;
+            if constexpr (kKeep) o.d0[j] = d;
             const float2 e = __ffma2_rn(x2[j], neg1, d);
             sq[j] = __fmul2_rn(e, e);
         }
-        err0 = error_sum(sq);
-        lo0 = hi0 = 0;
+        o.err0 = error_sum(sq);
         if constexpr (kPack) {
-            lo0 = __byte_perm(__float_as_uint(__fadd_rn(p4[0], 8388608.0f)), __float_as_uint(__fadd_rn(p4[1], 8388608.0f)), 0x5410);
-            hi0 = __byte_perm(__float_as_uint(__fadd_rn(p4[2], 8388608.0f)), __float_as_uint(__fadd_rn(p4[3], 8388608.0f)), 0x5410);
+            o.lo0 = __byte_perm(__float_as_uint(__fadd_rn(p4[0], 8388608.0f)), __float_as_uint(__fadd_rn(p4[1], 8388608.0f)), 0x5410);
+            o.hi0 = __byte_perm(__float_as_uint(__fadd_rn(p4[2], 8388608.0f)), __float_as_uint(__fadd_rn(p4[3], 8388608.0f)), 0x5410);
         }
+    }
+}
+
+// The same with IEEE divisions: any tensor scale, infinities and NaN.
+template <bool kPack, bool kKeep>
+__device__ __noinline__ void candidates_ieee(const float2 (&x2)[8], float gs, BlockCandidates<kPack, kKeep>& o) {
+    float s[kGroup], ax[kGroup];
+    float amax_s = 0.0f;
+    uint32_t sl = 0, sh = 0;                             // sign nibbles of elements 0..7 and 8..15
+#pragma unroll
+    for (int i = 0; i < kGroup; ++i) {
+        const float x = i & 1 ? x2[i >> 1].y : x2[i >> 1].x;
+        s[i] = __fdiv_rn(x, gs);
+        ax[i] = fabsf(x);
+        amax_s = fmaxf(amax_s, fabsf(s[i]));
+        // Sign bit of a nibble = (x < 0): dividing by the positive scales keeps the sign; -0 is not below zero.
+        if (x < 0.0f) (i < 8 ? sl : sh) |= 8u << (4 * (i & 7));
+    }
+    float d2[kGroup], d0[kGroup];
+    candidate<false, kPack, kKeep>(ax, s, amax_s, gs, o.lo2, o.hi2, o.byte2, o.sc2, o.err2, d2);
+    candidate<true, kPack, kKeep>(ax, s, amax_s, gs, o.lo0, o.hi0, o.byte0, o.sc0, o.err0, d0);
+    if constexpr (kPack) { o.lo2 |= sl; o.hi2 |= sh; }
+    if constexpr (kKeep) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            o.d2[j] = make_float2(x2[j].x < 0.0f ? -d2[2 * j] : d2[2 * j], x2[j].y < 0.0f ? -d2[2 * j + 1] : d2[2 * j + 1]);
+            o.d0[j] = make_float2(d0[2 * j], d0[2 * j + 1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float& v = h ? o.d0[j].y : o.d0[j].x;
+                if ((h ? x2[j].y : x2[j].x) < 0.0f) v = -v;
+            }
+        }
+    }
+}
+
+template <typename T, bool kPack, bool kKeep>
+__device__ __forceinline__ void block_candidates(const float2 (&x2)[8], float gs, float rgs, bool fast, BlockCandidates<kPack, kKeep>& o) {
+    if (fast) candidates_fast<sizeof(T) == 4>(x2, gs, rgs, o);
+    // a NaN (or a value whose quotient overflows) leaves the packed path with a NaN or an infinity in the error
+    if (!fast || !(__fadd_rn(o.err2, o.err0) < __int_as_float(0x7f800000))) {
+        float2 copy[8];                                  // copies: only these have addresses, o stays in registers
+        BlockCandidates<kPack, kKeep> t;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) copy[j] = x2[j];
+        candidates_ieee(copy, gs, t);
+        o = t;
+    }
+}
+
+// Tensor scale and whether the packed path gives the IEEE quotients of x / gs.  16-bit inputs: checked here by the
+// whole CTA for every significand the type has (128 or 1024 divisions); fp32 inputs: Markstein's condition on the
+// divisor, and a scale of at most 1 so that no quotient of a nonzero x rounds to zero (its sign would be lost).
+template <typename T>
+__device__ __forceinline__ bool tensor_scale(const float* amax_ptr, float& gs, float& rgs) {
+    const float amax = *amax_ptr;
+    gs = amax > 0.0f ? __fdiv_rn(amax, 2688.0f) : 1.0f;
+    rgs = __frcp_rn(gs);
+    if constexpr (sizeof(T) == 4) {
+        return gs > 8.7e-19f && gs <= 1.0f && (__float_as_uint(gs) & 0x7fffffu) != 0x7fffffu;
+    } else {
+        constexpr int kSig = Elem<T>::kDtype == MIXFP4_BF16 ? 128 : 1024;
+        bool ok = true;
+        for (int i = threadIdx.x; i < kSig; i += kThreads) {
+            const float v = 1.0f + static_cast<float>(i) * (1.0f / kSig);
+            ok = ok && __float_as_uint(div_rcp(v, gs, rgs)) == __float_as_uint(__fdiv_rn(v, gs));
+        }
+        return __syncthreads_and(ok) && gs > 8.7e-19f && gs < 1024.0f;
+    }
+}
+
+// Elements c0 .. c0 + 15 of a row (zeros past k); vec: 16-byte aligned rows; coherent: the tensor is being
+// overwritten in place.
+template <typename T>
+__device__ __forceinline__ void load_block(const T* src, int left, bool vec, bool coherent, float2 (&x2)[8]) {
+    float x[kGroup];
+    if (vec && left >= kGroup) {
+        constexpr int kWords = kGroup * sizeof(T) / 16;
+        uint4 w[kWords];
+#pragma unroll
+        for (int j = 0; j < kWords; ++j) {
+            const uint4* p = reinterpret_cast<const uint4*>(src) + j;
+            w[j] = coherent ? *p : __ldg(p);
+        }
+        const T* e = reinterpret_cast<const T*>(w);
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) x[i] = Elem<T>::load(e + i);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) x[i] = i < left ? Elem<T>::load(src + i) : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x2[j] = make_float2(x[2 * j], x[2 * j + 1]);
+}
+
+// The chosen candidate's dequantized values, rounded to T.  16-bit types: both candidates as packed pairs, the
+// E0M3 pair takes its signs from the E2M1 pair (a negative element that rounds to zero gives -0 in either format).
+template <typename T, bool kPack>
+__device__ __forceinline__ void store_block(T* out, int left, bool vec, bool use_e0, const BlockCandidates<kPack, true>& o) {
+    T vals[kGroup];
+    if constexpr (sizeof(T) == 2) {
+        uint32_t* v = reinterpret_cast<uint32_t*>(vals);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            T p2[2] = {Elem<T>::round(o.d2[j].x), Elem<T>::round(o.d2[j].y)};
+            T p0[2] = {Elem<T>::round(o.d0[j].x), Elem<T>::round(o.d0[j].y)};
+            const uint32_t w2 = *reinterpret_cast<const uint32_t*>(p2), w0 = *reinterpret_cast<const uint32_t*>(p0);
+            v[j] = use_e0 ? (w0 | (w2 & 0x80008000u)) : w2;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            vals[2 * j] = use_e0 ? __uint_as_float(__float_as_uint(o.d0[j].x) | (__float_as_uint(o.d2[j].x) & 0x80000000u)) : o.d2[j].x;
+            vals[2 * j + 1] = use_e0 ? __uint_as_float(__float_as_uint(o.d0[j].y) | (__float_as_uint(o.d2[j].y) & 0x80000000u)) : o.d2[j].y;
+        }
+    }
+    if (vec && left >= kGroup) {
+        constexpr int kWords = kGroup * sizeof(T) / 16;
+#pragma unroll
+        for (int j = 0; j < kWords; ++j) reinterpret_cast<uint4*>(out)[j] = reinterpret_cast<const uint4*>(vals)[j];
+    } else {
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i)
+            if (i < left) out[i] = vals[i];
     }
 }
 
@@ -429,6 +570,15 @@ __global__ void selftest_division_kernel(unsigned long long* mismatches) {
         bad += __float_as_uint(q2.x) != __float_as_uint(__fdiv_rn(a, b));
         bad += __float_as_uint(q2.y) != __float_as_uint(__fdiv_rn(-a * 0.37f, b));
     }
+    // two corrections, any divisor: 16 divisors per dividend, spread over all significands by a multiplicative hash
+    for (uint32_t d = 0; d < 16; ++d) {
+        const uint32_t sig = ((i * 16u + d) * 2654435761u) >> 9;
+        if (sig == 0x7fffffu) continue;
+        const float b = __uint_as_float(0x38000000u | sig), r = __frcp_rn(b);
+        const float2 q2 = div_rcp2_twice(make_float2(a, -a * 0.37f), make_float2(-b, -b), make_float2(r, r));
+        bad += __float_as_uint(q2.x) != __float_as_uint(__fdiv_rn(a, b));
+        bad += __float_as_uint(q2.y) != __float_as_uint(__fdiv_rn(-a * 0.37f, b));
+    }
     if (bad) atomicAdd(mismatches, bad);
 }
 
@@ -465,24 +615,11 @@ __global__ void __launch_bounds__(kThreads, (kPack && !kDequant) ? 3 : 2) quanti
     // a kernel launched behind this one with programmatic dependent launch (the W4A4 GEMM) may set itself up
     // while this grid runs; it waits for this grid's end before it reads the outputs
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");       // the pass that found the maximum (a no-op otherwise)
     const int lane = threadIdx.x & 31;
     const int warp_in_cta = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // provably warp-uniform
-    const float amax = *a.amax;
-    const float gs = amax > 0.0f ? __fdiv_rn(amax, 2688.0f) : 1.0f;
-    const float rgs = __frcp_rn(gs);
-    // The reciprocal form of x / gs is used only if it gives the IEEE quotient for every
-    // significand the 16-bit input type has (checked here by the whole CTA, 128 or 1024
-    // divisions); fp32 inputs and extreme tensor scales take the IEEE path.
-    bool fast = sizeof(T) == 2 && gs > 8.7e-19f && gs < 1024.0f;
-    {
-        constexpr int kSig = sizeof(T) == 2 ? (Elem<T>::kDtype == MIXFP4_BF16 ? 128 : 1024) : 0;
-        bool ok = true;
-        for (int i = threadIdx.x; i < kSig; i += kThreads) {
-            const float v = 1.0f + static_cast<float>(i) * (1.0f / kSig);
-            ok = ok && __float_as_uint(div_rcp(v, gs, rgs)) == __float_as_uint(__fdiv_rn(v, gs));
-        }
-        fast = __syncthreads_and(ok) && fast;
-    }
+    float gs, rgs;
+    const bool fast = tensor_scale<T>(a.amax, gs, rgs);
     if (blockIdx.x == 0 && threadIdx.x == 0 && a.global_scale) *a.global_scale = gs;
 
     // (row, chunk) of this warp's items: one division here, carries in the loop
@@ -506,100 +643,29 @@ __global__ void __launch_bounds__(kThreads, (kPack && !kDequant) ? 3 : 2) quanti
             use_e0 = (a.fmt[row * (a.blocks_pad / 8) + (blk >> 3)] >> (blk & 7)) & 1;
 
         if (real) {
-            const T* xr = static_cast<const T*>(a.x) + row * a.ldx;
             const int64_t c0 = blk * kGroup;
-            float x[kGroup];
-            if (a.vec_in && c0 + kGroup <= a.k) {
-                constexpr int kWords = kGroup * sizeof(T) / 16;
-                uint4 w[kWords];
-#pragma unroll
-                for (int j = 0; j < kWords; ++j) {
-                    const uint4* src = reinterpret_cast<const uint4*>(xr + c0) + j;
-                    w[j] = a.in_place ? *src : __ldg(src);
-                }
-                const T* e = reinterpret_cast<const T*>(w);
-#pragma unroll
-                for (int i = 0; i < kGroup; ++i) x[i] = Elem<T>::load(e + i);
-            } else {
-#pragma unroll
-                for (int i = 0; i < kGroup; ++i) x[i] = c0 + i < a.k ? Elem<T>::load(xr + c0 + i) : 0.0f;
-            }
-
-            uint32_t lo2, hi2, b2, lo0, hi0, b0;
-            float sc2, sc0, err2, err0;
-            float d2[kGroup], d0[kGroup];
-            uint32_t sl = 0, sh = 0;                     // sign nibbles of elements 0..7 and 8..15
-            if (fast) {
-                float2 x2[8], dd2[8], dd0[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) x2[j] = make_float2(x[2 * j], x[2 * j + 1]);
-                candidates_fast<kPack, kDequant>(x2, gs, rgs, lo2, hi2, b2, sc2, err2, dd2, lo0, hi0, b0, sc0, err0, dd0);
-                if constexpr (kDequant) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        d2[2 * j] = fabsf(dd2[j].x); d2[2 * j + 1] = fabsf(dd2[j].y);
-                        d0[2 * j] = fabsf(dd0[j].x); d0[2 * j + 1] = fabsf(dd0[j].y);
-                    }
-                }
-                sl = lo2 & 0x88888888u;                  // the FP4 unit kept the quotients' signs
-                sh = hi2 & 0x88888888u;
-            } else {
-                float s[kGroup], ax[kGroup];
-                float amax_s = 0.0f;
-#pragma unroll
-                for (int i = 0; i < kGroup; ++i) {
-                    s[i] = __fdiv_rn(x[i], gs);
-                    ax[i] = fabsf(x[i]);
-                    amax_s = fmaxf(amax_s, fabsf(s[i]));
-                }
-                candidate<false, false, kPack, kDequant>(ax, s, amax_s, gs, lo2, hi2, b2, sc2, err2, d2);
-                candidate<true, false, kPack, kDequant>(ax, s, amax_s, gs, lo0, hi0, b0, sc0, err0, d0);
-                if constexpr (kPack) {
-                    // Sign bit of a nibble = (n < 0) = (x < 0): dividing by the positive scales keeps the sign and
-                    // never reaches zero from a nonzero x; x = -0 gives n = -0, which is not below zero.
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        if (x[i] < 0.0f) sl |= 8u << (4 * i);
-                        if (x[i + 8] < 0.0f) sh |= 8u << (4 * i);
-                    }
-                }
-            }
+            const int left = (int)min((int64_t)kGroup, a.k - c0);
+            float2 x2[8];
+            load_block(static_cast<const T*>(a.x) + row * a.ldx + c0, left, a.vec_in, a.in_place, x2);
+            BlockCandidates<kPack, kDequant> o;
+            block_candidates<T>(x2, gs, rgs, fast, o);
             if (a.mode != MIXFP4_MODE_GIVEN)
-                use_e0 = a.mode == MIXFP4_MODE_ORACLE16 ? (err0 < err2) : (a.mode == MIXFP4_MODE_ALL_E0M3);
+                use_e0 = a.mode == MIXFP4_MODE_ORACLE16 ? (o.err0 < o.err2) : (a.mode == MIXFP4_MODE_ALL_E0M3);
 
             if (a.any_stats) {
                 const int64_t g = row * a.groups + blk;
-                if (a.e2_err) a.e2_err[g] = err2;
-                if (a.e0_err) a.e0_err[g] = err0;
-                if (a.e2_scale) a.e2_scale[g] = sc2;
-                if (a.e0_scale) a.e0_scale[g] = sc0;
+                if (a.e2_err) a.e2_err[g] = o.err2;
+                if (a.e0_err) a.e0_err[g] = o.err0;
+                if (a.e2_scale) a.e2_scale[g] = o.sc2;
+                if (a.e0_scale) a.e0_scale[g] = o.sc0;
             }
-
             if constexpr (kPack) {
-                lo = (use_e0 ? lo0 : lo2) | sl;
-                hi = (use_e0 ? hi0 : hi2) | sh;
-                scale_byte = use_e0 ? b0 : b2;
+                lo = use_e0 ? o.lo0 | (o.lo2 & 0x88888888u) : o.lo2;
+                hi = use_e0 ? o.hi0 | (o.hi2 & 0x88888888u) : o.hi2;
+                scale_byte = use_e0 ? o.byte0 : o.byte2;
             }
-
-            if constexpr (kDequant) {
-                T* out = static_cast<T*>(a.dequant) + row * a.ld_dequant + c0;
-                T vals[kGroup];
-#pragma unroll
-                for (int i = 0; i < kGroup; ++i) {
-                    const float mag = use_e0 ? d0[i] : d2[i];
-                    vals[i] = Elem<T>::round(x[i] < 0.0f ? -mag : mag);
-                }
-                if (a.vec_out && c0 + kGroup <= a.k) {
-                    constexpr int kWords = kGroup * sizeof(T) / 16;
-#pragma unroll
-                    for (int j = 0; j < kWords; ++j)
-                        reinterpret_cast<uint4*>(out)[j] = reinterpret_cast<const uint4*>(vals)[j];
-                } else {
-#pragma unroll
-                    for (int i = 0; i < kGroup; ++i)
-                        if (c0 + i < a.k) out[i] = vals[i];
-                }
-            }
+            if constexpr (kDequant)
+                store_block(static_cast<T*>(a.dequant) + row * a.ld_dequant + c0, left, a.vec_out, use_e0, o);
         }
 
         if constexpr (kPack) {
@@ -614,6 +680,146 @@ __global__ void __launch_bounds__(kThreads, (kPack && !kDequant) ? 3 : 2) quanti
                 a.fmt[row * (a.blocks_pad / 8) + fmt_col] = static_cast<uint8_t>(bits >> (8 * lane));
         }
       }
+    }
+}
+
+// Quantizes straight into the stream layout (decode.cuh): an item is a quarter of a chunk, four rows x 128 K, so that
+// a warp reads 256-byte (16-bit types) runs of four rows and writes 256 bytes of codes and one whole sector of scale bytes.
+// Rows past the tensor and blocks past K get what an all-zero block quantizes to.  CTA 0 also writes the weight's
+// decode table.  Bound by instruction issue like the kernel above.  Loading a rotated 14336 x 4096 bf16 projection
+// (rotation with the maximum in the same pass, this kernel, nothing else): 169 us, against 220 us for rotation, amax,
+// canonical quantizer, repack and table launch.
+struct StreamQuantArgs {
+    const void* x;
+    int64_t rows, k, ldx, groups, subs, items;       // items = row tiles * subs * 4
+    int mode;
+    bool vec_in;
+    const float* amax;
+    uint8_t* chunks;
+    float* global_scale;
+    uint4* lut;                                       // optional: mixfp4_decode_table_wide's image
+};
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 3) quantize_stream_kernel(const StreamQuantArgs a) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    const int warp_in_cta = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // provably warp-uniform
+    float gs, rgs;
+    const bool fast = tensor_scale<T>(a.amax, gs, rgs);
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) *a.global_scale = gs;
+        if (a.lut) {
+            const int e = threadIdx.x;
+            const uint4 v = make_lut_entry(e & 127, e >> 7, gs);
+            a.lut[e] = v;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a.lut[256 + e * 8 + j] = v;
+        }
+    }
+    const int64_t step = (int64_t)gridDim.x * kWarpsPerCta;
+    for (int64_t item = (int64_t)blockIdx.x * kWarpsPerCta + warp_in_cta; item < a.items; item += step) {
+        const int64_t chunk = item >> 2, tile = chunk / a.subs, sub = chunk - tile * a.subs;
+        const int q = (int)(item & 3);
+        const int64_t row = tile * kChunkRows + q * 4 + (lane >> 3), blk = sub * 8 + (lane & 7);
+        uint32_t lo = 0, hi = 0, scale_byte = 0x01;
+        if (row < a.rows && blk < a.groups) {
+            const int64_t c0 = blk * kGroup;
+            float2 x2[8];
+            load_block(static_cast<const T*>(a.x) + row * a.ldx + c0, (int)min((int64_t)kGroup, a.k - c0), a.vec_in, false, x2);
+            BlockCandidates<true, false> o;
+            block_candidates<T>(x2, gs, rgs, fast, o);
+            const bool use_e0 = a.mode == MIXFP4_MODE_ORACLE16 ? (o.err0 < o.err2) : (a.mode == MIXFP4_MODE_ALL_E0M3);
+            lo = codes_to_kernel_layout(use_e0 ? o.lo0 | (o.lo2 & 0x88888888u) : o.lo2);
+            hi = codes_to_kernel_layout(use_e0 ? o.hi0 | (o.hi2 & 0x88888888u) : o.hi2);
+            scale_byte = use_e0 ? (o.byte0 | 0x80u) : o.byte2;
+        }
+        uint8_t* dst = a.chunks + chunk * kChunkBytes;
+        *reinterpret_cast<uint2*>(dst + q * 256 + lane * 8) = make_uint2(lo, hi);
+        dst[kChunkCodeBytes + q * 32 + lane] = static_cast<uint8_t>(scale_byte);
+    }
+}
+
+// Fake quantization with one format per region of R x G blocks (powers of two, R <= 64, G <= 4), in one pass: a
+// CTA takes a tile of max(8, R) rows by as many block columns as make 256 blocks, a thread one block; both candidates
+// stay in registers while the errors of the tile's regions are summed in shared memory in the order of
+// select_regions_kernel (so the decisions are the same bits), then the chosen one is stored.  The separate passes
+// quantized every block twice and moved the errors through memory (3001 x 4100 fp32, 8 x 64 regions: 133 us with
+// them and IEEE divisions, 49 us with this kernel and the packed fp32 path).
+struct RegionArgs {
+    const void* x;
+    int64_t rows, k, ldx, groups, tiles_g, tiles;
+    int r_log2, g_log2, tg_log2;                      // region rows, region groups, tile columns
+    bool vec_in, vec_out;
+    const float* amax;
+    void* out;
+    int64_t ldo;
+};
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 2) fake_regions_kernel(const RegionArgs a) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float e2[kThreads], e0[kThreads], s2[kThreads], s0[kThreads];
+    __shared__ uint8_t pick[kThreads];
+    float gs, rgs;
+    const bool fast = tensor_scale<T>(a.amax, gs, rgs);
+    const int tg = 1 << a.tg_log2, tr = kThreads >> a.tg_log2, rl = a.r_log2, gl = a.g_log2;
+    const int r = threadIdx.x >> a.tg_log2, g = threadIdx.x & (tg - 1);
+    const int rg_log2 = a.tg_log2 - gl;               // regions along the tile's columns
+    for (int64_t t = blockIdx.x; t < a.tiles; t += gridDim.x) {
+        const int64_t tile_r = t / a.tiles_g, tile_g = t - tile_r * a.tiles_g;
+        const int64_t row = tile_r * tr + r, blk = tile_g * tg + g, c0 = blk * kGroup;
+        const bool real = row < a.rows && blk < a.groups;
+        const int left = real ? (int)min((int64_t)kGroup, a.k - c0) : 0;
+        BlockCandidates<false, true> o;
+        o.err2 = o.err0 = 0.0f;                       // cells past the tensor's edge count as zero
+        if (real) {
+            float2 x2[8];
+            load_block(static_cast<const T*>(a.x) + row * a.ldx + c0, left, a.vec_in, false, x2);
+            block_candidates<T>(x2, gs, rgs, fast, o);
+        }
+        e2[threadIdx.x] = o.err2;
+        e0[threadIdx.x] = o.err0;
+        __syncthreads();
+        if (gl > 0) {
+            // a row of a region left to right, then the rows top to bottom
+            if ((int)threadIdx.x < kThreads >> gl) {
+                const int first = threadIdx.x << gl;
+                float t2 = 0.0f, t0 = 0.0f;
+                for (int i = 0; i < 1 << gl; ++i) { t2 = __fadd_rn(t2, e2[first + i]); t0 = __fadd_rn(t0, e0[first + i]); }
+                s2[threadIdx.x] = t2;
+                s0[threadIdx.x] = t0;
+            }
+            __syncthreads();
+        }
+        if ((int)threadIdx.x < kThreads >> (rl + gl)) {
+            const float* c2 = gl > 0 ? s2 : e2;
+            const float* c0p = gl > 0 ? s0 : e0;
+            const int rr = threadIdx.x >> rg_log2, cg = threadIdx.x & ((1 << rg_log2) - 1);
+            const int first = ((rr << rl) << rg_log2) + cg, stride = 1 << rg_log2, n = 1 << rl;
+            float sum2 = 0.0f, sum0 = 0.0f;
+            if (gl == 0 && tile_g * tg + cg >= a.groups / 32 * 32) {
+                // one-block columns after the last whole 32: four accumulators (see select_regions_kernel)
+                float a2[4] = {0.0f, 0.0f, 0.0f, 0.0f}, a0[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                for (int i = 0; i < n; i += 4)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (i + q < n) {
+                            a2[q] = __fadd_rn(a2[q], c2[first + (i + q) * stride]);
+                            a0[q] = __fadd_rn(a0[q], c0p[first + (i + q) * stride]);
+                        }
+                sum2 = __fadd_rn(__fadd_rn(__fadd_rn(a2[0], a2[1]), a2[2]), a2[3]);
+                sum0 = __fadd_rn(__fadd_rn(__fadd_rn(a0[0], a0[1]), a0[2]), a0[3]);
+            } else {
+                for (int i = 0; i < n; ++i) {
+                    sum2 = __fadd_rn(sum2, c2[first + i * stride]);
+                    sum0 = __fadd_rn(sum0, c0p[first + i * stride]);
+                }
+            }
+            pick[threadIdx.x] = sum0 < sum2;
+        }
+        __syncthreads();
+        if (real)
+            store_block(static_cast<T*>(a.out) + row * a.ldo + c0, left, a.vec_out, pick[((r >> rl) << rg_log2) + (g >> gl)] != 0, o);
+        // no barrier here: the next tile's sums are read after its own barrier, and `pick` is rewritten after it too
     }
 }
 
@@ -901,9 +1107,26 @@ __global__ void __launch_bounds__(kThreads) fill_format_kernel(const double* __r
 
 namespace mixfp4 {
 namespace {
+// after_amax: the kernel launched just before on this stream found the maximum and signals its dependents early;
+// this launch may then start under its tail (the kernels wait for that grid's end first thing).
+template <typename Args>
+int launch_after(void (*kernel)(const Args), int64_t ctas, bool after_amax, cudaStream_t st, const Args& a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = after_amax ? 1 : 0;
+    MIXFP4_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, a));
+    return MIXFP4_OK;
+}
+
 int launch_quantize(const void* x, int dtype, int64_t rows, int64_t k, int64_t ldx, int mode, const float* amax,
                     uint8_t* codes, uint8_t* scales, uint8_t* fmt, float* global_scale, float* e2_err, float* e0_err,
-                    float* e2_scale, float* e0_scale, void* dequant, int64_t ld_dequant, cudaStream_t st) {
+                    float* e2_scale, float* e0_scale, void* dequant, int64_t ld_dequant, bool after_amax, cudaStream_t st) {
     QuantArgs a;
     a.x = x; a.rows = rows; a.k = k; a.ldx = ldx;
     a.groups = (k + kGroup - 1) / kGroup;
@@ -922,9 +1145,9 @@ int launch_quantize(const void* x, int dtype, int64_t rows, int64_t k, int64_t l
     if (ctas > 148 * 6) ctas = 148 * 6;            // the warps stride over the (row, chunk) items
 #define MIXFP4_LAUNCH_QUANTIZE(T)                                                                       \
     do {                                                                                                \
-        if (codes && dequant) quantize_kernel<T, true, true><<<(unsigned)ctas, kThreads, 0, st>>>(a);    \
-        else if (codes) quantize_kernel<T, true, false><<<(unsigned)ctas, kThreads, 0, st>>>(a);         \
-        else quantize_kernel<T, false, true><<<(unsigned)ctas, kThreads, 0, st>>>(a);                    \
+        if (codes && dequant) return launch_after(quantize_kernel<T, true, true>, ctas, after_amax, st, a);  \
+        if (codes) return launch_after(quantize_kernel<T, true, false>, ctas, after_amax, st, a);           \
+        return launch_after(quantize_kernel<T, false, true>, ctas, after_amax, st, a);                      \
     } while (0)
     switch (dtype) {
         case MIXFP4_BF16: MIXFP4_LAUNCH_QUANTIZE(__nv_bfloat16); break;
@@ -932,14 +1155,13 @@ int launch_quantize(const void* x, int dtype, int64_t rows, int64_t k, int64_t l
         default: MIXFP4_LAUNCH_QUANTIZE(float);
     }
 #undef MIXFP4_LAUNCH_QUANTIZE
-    return check_launch("quantize_kernel");
 }
 }  // namespace
 
 int fake_quantize_with_amax(const void* x, int dtype, int64_t rows, int64_t k, int64_t ldx, int mode, const float* amax,
                             void* y, int64_t ldy, cudaStream_t st) {
     return launch_quantize(x, dtype, rows, k, ldx, mode, amax, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                           nullptr, nullptr, y, ldy, st);
+                           nullptr, nullptr, y, ldy, true, st);
 }
 }  // namespace mixfp4
 
@@ -953,7 +1175,7 @@ extern "C" int mixfp4_quantize(const void* x, int dtype, int64_t rows, int64_t k
     if (mode < MIXFP4_MODE_ORACLE16 || mode > MIXFP4_MODE_GIVEN) return MIXFP4_E_MODE;
     if (!aligned(codes, 8)) return MIXFP4_E_ALIGN;
     return launch_quantize(x, dtype, rows, k, ldx, mode, amax, codes, scales, fmt, global_scale, e2_err, e0_err,
-                           e2_scale, e0_scale, dequant, ld_dequant, static_cast<cudaStream_t>(stream));
+                           e2_scale, e0_scale, dequant, ld_dequant, false, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mixfp4_fake_quantize(const void* x, int dtype, int64_t rows, int64_t k, int64_t ldx, int mode,
@@ -967,7 +1189,64 @@ extern "C" int mixfp4_fake_quantize(const void* x, int dtype, int64_t rows, int6
     const int rc = mixfp4_amax(x, dtype, rows, k, ldx, amax, stream);
     if (rc != MIXFP4_OK) return rc;
     return launch_quantize(x, dtype, rows, k, ldx, mode, amax, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                           nullptr, nullptr, y, ldy, static_cast<cudaStream_t>(stream));
+                           nullptr, nullptr, y, ldy, true, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mixfp4_fake_quantize_regions(const void* x, int dtype, int64_t rows, int64_t k, int64_t ldx,
+                                            int region_rows, int region_groups, float* amax, void* y, int64_t ldy,
+                                            void* stream) {
+    if (!x || !amax || !y) return MIXFP4_E_NULL;
+    if (rows <= 0 || k <= 0 || ldx < k || ldy < k || y == x || region_rows <= 0) return MIXFP4_E_SHAPE;
+    if (dtype < MIXFP4_BF16 || dtype > MIXFP4_F32) return MIXFP4_E_DTYPE;
+    if (region_rows > 64 || (region_rows & (region_rows - 1))) return MIXFP4_E_MODE;
+    if (region_groups != 1 && region_groups != 2 && region_groups != 4) return MIXFP4_E_MODE;
+    if (region_groups == 1 && region_rows < 2) return MIXFP4_E_MODE;         // 1 x 1 is the per-block mode
+    RegionArgs a;
+    a.groups = (k + kGroup - 1) / kGroup;
+    // with a single region along K the reference's reduction takes another order (not reproduced)
+    if (region_rows > 1 && (a.groups + region_groups - 1) / region_groups == 1) return MIXFP4_E_MODE;
+    const int rc = mixfp4_amax(x, dtype, rows, k, ldx, amax, stream);
+    if (rc != MIXFP4_OK) return rc;
+    a.x = x; a.rows = rows; a.k = k; a.ldx = ldx; a.amax = amax; a.out = y; a.ldo = ldy;
+    a.r_log2 = 31 - __builtin_clz((unsigned)region_rows);
+    a.g_log2 = 31 - __builtin_clz((unsigned)region_groups);
+    const int tr_log2 = a.r_log2 < 3 ? 3 : a.r_log2;
+    a.tg_log2 = 8 - tr_log2;
+    a.tiles_g = (a.groups + (1 << a.tg_log2) - 1) >> a.tg_log2;
+    a.tiles = ((rows + (1 << tr_log2) - 1) >> tr_log2) * a.tiles_g;
+    a.vec_in = rows_vectorizable(x, ldx, dtype);
+    a.vec_out = rows_vectorizable(y, ldy, dtype);
+    const int64_t ctas = a.tiles < 148 * 4 ? a.tiles : 148 * 4;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    switch (dtype) {
+        case MIXFP4_BF16: return launch_after(fake_regions_kernel<__nv_bfloat16>, ctas, true, st, a);
+        case MIXFP4_F16: return launch_after(fake_regions_kernel<__half>, ctas, true, st, a);
+        default: return launch_after(fake_regions_kernel<float>, ctas, true, st, a);
+    }
+}
+
+extern "C" int mixfp4_quantize_stream(const void* x, int dtype, int64_t rows, int64_t k, int64_t ldx, int mode,
+                                      const float* amax, uint8_t* chunks, float* global_scale, void* lut, void* stream) {
+    if (!x || !amax || !chunks || !global_scale) return MIXFP4_E_NULL;
+    if (rows <= 0 || k <= 0 || ldx < k) return MIXFP4_E_SHAPE;
+    if (dtype < MIXFP4_BF16 || dtype > MIXFP4_F32) return MIXFP4_E_DTYPE;
+    if (mode < MIXFP4_MODE_ORACLE16 || mode > MIXFP4_MODE_ALL_E0M3) return MIXFP4_E_MODE;
+    if (!aligned(chunks, 16) || (lut && !aligned(lut, 16))) return MIXFP4_E_ALIGN;
+    StreamQuantArgs a;
+    a.x = x; a.rows = rows; a.k = k; a.ldx = ldx; a.mode = mode; a.amax = amax;
+    a.groups = (k + kGroup - 1) / kGroup;
+    a.subs = padded_k(k) / kChunkK;
+    a.items = stream_tiles(rows) * a.subs * 4;
+    a.vec_in = rows_vectorizable(x, ldx, dtype);
+    a.chunks = chunks; a.global_scale = global_scale; a.lut = static_cast<uint4*>(lut);
+    int64_t ctas = (a.items + kWarpsPerCta - 1) / kWarpsPerCta;
+    if (ctas > 148 * 6) ctas = 148 * 6;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    switch (dtype) {
+        case MIXFP4_BF16: return launch_after(quantize_stream_kernel<__nv_bfloat16>, ctas, false, st, a);
+        case MIXFP4_F16: return launch_after(quantize_stream_kernel<__half>, ctas, false, st, a);
+        default: return launch_after(quantize_stream_kernel<float>, ctas, false, st, a);
+    }
 }
 
 extern "C" int mixfp4_dequant(const uint8_t* codes, const uint8_t* scales, const uint8_t* fmt,

@@ -16,7 +16,7 @@ from torch import nn
 from . import _native as nat
 from . import rotation as _rotation
 from .quant import (HIGH_PRECISION_MODES, PackedWeight, _MODE_CODE, fake_quantize_activations, normalize_region,
-                    quantize_packed, region_shape)
+                    quantize_packed, quantize_stream, region_shape)
 
 GEMV_MAX_M = 16
 _workspaces: dict[tuple, torch.Tensor] = {}
@@ -233,9 +233,15 @@ class MixFP4Linear(nn.Module):
         w = linear.weight.detach().to(device)
         if w.dtype not in nat.DTYPE_CODE:
             w = w.to(torch.bfloat16)
+        amax = None
         if rotation is not None:
-            w = _rotation.apply_transform(w, rotation)
-        packed, _, _ = quantize_packed(w, mode=mode, rotation=rotation)
+            amax = torch.empty(1, dtype=torch.float32, device=device)
+            rotated = _rotation.apply_transform(w, rotation, amax=amax)
+            w, amax = rotated, (amax if rotated is not w else None)
+        if mode in _MODE_CODE:
+            packed = quantize_stream(w, mode=mode, amax=amax, rotation=rotation)
+        else:
+            packed, _, _ = quantize_packed(w, mode=mode, amax=amax, rotation=rotation)
         bias = None if linear.bias is None else linear.bias.detach().to(device)
         return cls(packed, bias, activation_mode)
 

@@ -336,6 +336,29 @@ def quantize_packed(x: torch.Tensor, *, mode: str = "oracle16", amax: torch.Tens
     return PackedWeight(codes, scales, fmt, gs, rows, k, rotation), dq, stats
 
 
+def quantize_stream(x: torch.Tensor, *, mode: str = "oracle16", amax: torch.Tensor | None = None,
+                    rotation: str | None = None) -> PackedWeight:
+    """``quantize_packed(x, mode=...)[0].to_stream_layout()`` for a per-block or whole-tensor mode without the
+    canonical arrays in between: the quantizer writes the stream layout and the decode table itself."""
+    if mode not in _MODE_CODE:
+        raise ValueError(f"unsupported mode {mode!r}")
+    x2 = _as_rows(x)
+    rows, k = x2.shape
+    dev = x2.device
+    if amax is None:
+        amax = tensor_amax(x2)
+    lib = nat.lib()
+    chunks = torch.empty(lib.mixfp4_stream_bytes(rows, k), dtype=torch.uint8, device=dev)
+    lut = torch.empty(nat.WIDE_TABLE_BYTES, dtype=torch.uint8, device=dev)
+    gs = torch.empty(1, dtype=torch.float32, device=dev)
+    with torch.cuda.device(dev):
+        st = lib.mixfp4_quantize_stream(x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], rows, k, x2.stride(0), _MODE_CODE[mode],
+                                        amax.data_ptr(), chunks.data_ptr(), gs.data_ptr(), lut.data_ptr(),
+                                        nat.stream_ptr(dev))
+    nat.check("mixfp4_quantize_stream", st)
+    return PackedWeight(chunks, torch.empty(0, dtype=torch.uint8, device=dev), None, gs, rows, k, rotation, "stream", lut)
+
+
 def _codebook(x: torch.Tensor, e0m3: bool) -> torch.Tensor:
     if not torch.is_floating_point(x):
         raise TypeError("x must be floating point")
@@ -514,28 +537,37 @@ def fake_quantize_activations(x: torch.Tensor, mode: str = "oracle16", *, in_pla
     (project_quant/modeling.py:669-705): ``quant_mixfp4_granularity(x, format_region=mode,
     operand_role="activation_a")`` -- x's own global scale, K16 block scales, one format per
     block or per activation region (m4k64 ...), dequantized back to x.dtype.  x: CUDA tensor
-    [..., K].  Per-block and whole-tensor modes run as one amax and one quantizer launch with
-    no packed outputs (``mixfp4_fake_quantize``); region modes take the three-pass route.
+    [..., K].  All modes but "layer" run as one amax and one quantizer launch with no packed outputs
+    (``mixfp4_fake_quantize``, ``mixfp4_fake_quantize_regions``); "layer" takes the three-pass route.
     in_place=True overwrites x (it must then be contiguous along K with a dense row stride)."""
     mode = normalize_region(mode, "activation_a")
     if mode in HIGH_PRECISION_MODES:
         return x
-    region = region_shape(mode, "activation_a")
+    return _fake_quantize(x, mode, region_shape(mode, "activation_a"), in_place)
+
+
+def _fake_quantize(x: torch.Tensor, mode: str, region: tuple[int, int] | None, in_place: bool = False) -> torch.Tensor:
+    """quantize_packed(x, mode, want_dequant=True)[1] in x's shape without packed outputs."""
     x2 = _as_rows(x)
-    if region is not None:
+    rows, k = x2.shape
+    if region is not None and region[1] == 0:             # "layer" decides on the whole tensor's error sums
         dq = quantize_packed(x2, mode=mode, want_dequant=True, region=region)[1]
         if in_place:
             x.copy_(dq.reshape(x.shape))
             return x
         return dq.reshape(x.shape)
-    aliases_input = x2.data_ptr() == x.data_ptr() and x2.stride(-1) == 1
+    if region is not None and region[0] > 1 and -(-((k + 15) // 16) // region[1]) == 1:
+        raise NotImplementedError("coarse regions over several rows need more than one region along K")
+    aliases_input = region is None and x2.data_ptr() == x.data_ptr() and x2.stride(-1) == 1
     out = x2 if in_place and aliases_input else torch.empty_like(x2, memory_format=torch.contiguous_format)
     amax = torch.empty(1, dtype=torch.float32, device=x2.device)
+    head = (x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], rows, k, x2.stride(0))
+    tail = (amax.data_ptr(), out.data_ptr(), out.stride(0), nat.stream_ptr(x2.device))
     with torch.cuda.device(x2.device):
-        st = nat.lib().mixfp4_fake_quantize(x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], x2.shape[0], x2.shape[1],
-                                            x2.stride(0), _MODE_CODE[mode], amax.data_ptr(), out.data_ptr(),
-                                            out.stride(0), nat.stream_ptr(x2.device))
-    nat.check("mixfp4_fake_quantize", st)
+        if region is None:
+            nat.check("mixfp4_fake_quantize", nat.lib().mixfp4_fake_quantize(*head, _MODE_CODE[mode], *tail))
+        else:
+            nat.check("mixfp4_fake_quantize_regions", nat.lib().mixfp4_fake_quantize_regions(*head, *region, *tail))
     if in_place and not aliases_input:
         x.copy_(out.reshape(x.shape))
         return x
@@ -628,12 +660,13 @@ def quant_mixfp4_granularity(
     if transform is not None:
         working = _rotation.apply_transform(working, transform)
 
-    packed, dq, stats = quantize_packed(working, mode=mode, want_dequant=True, want_stats=return_stats, region=region)
+    if not return_stats:
+        dequant = _fake_quantize(working, mode, region)
+        return dequant.to(x.device) if host_input else dequant
+    packed, dq, stats = quantize_packed(working, mode=mode, want_dequant=True, want_stats=True, region=region)
     dequant = dq.reshape(working.shape)
     if host_input:
         dequant = dequant.to(x.device)
-    if not return_stats:
-        return dequant
 
     e2e, e0e = stats["e2_errors"], stats["e0_errors"]
     ids = packed.format_ids()

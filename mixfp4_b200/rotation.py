@@ -67,7 +67,7 @@ def _device_signs(size: int, seed: int, device) -> torch.Tensor:
 
 
 def _run_fwht(x: torch.Tensor, size: int, signs: torch.Tensor | None, stagewise: bool,
-              out: torch.Tensor | None = None) -> torch.Tensor:
+              out: torch.Tensor | None = None, amax: torch.Tensor | None = None) -> torch.Tensor:
     if x.dtype not in nat.DTYPE_CODE:
         raise TypeError("x must be bfloat16, float16 or float32")
     if size not in _SUPPORTED_SIZES:
@@ -79,9 +79,13 @@ def _run_fwht(x: torch.Tensor, size: int, signs: torch.Tensor | None, stagewise:
     k = src.shape[-1]
     rows = src.numel() // k
     dst = out if out is not None else torch.empty_like(src)
+    args = (src.data_ptr(), dst.data_ptr(), nat.DTYPE_CODE[src.dtype], rows, k, k, k, size, nat.ptr(signs),
+            1 if stagewise else 0)
     with torch.cuda.device(src.device):
-        st = nat.lib().mixfp4_fwht(src.data_ptr(), dst.data_ptr(), nat.DTYPE_CODE[src.dtype], rows, k, k, k,
-                                   size, nat.ptr(signs), 1 if stagewise else 0, nat.stream_ptr(src.device))
+        if amax is None:
+            st = nat.lib().mixfp4_fwht(*args, nat.stream_ptr(src.device))
+        else:                                       # float32 [1] on the device: the largest magnitude of the result
+            st = nat.lib().mixfp4_fwht_amax(*args, amax.data_ptr(), nat.stream_ptr(src.device))
     nat.check("mixfp4_fwht", st)
     return dst.to(x.device) if host else dst
 
@@ -94,11 +98,14 @@ def fwht(x: torch.Tensor) -> torch.Tensor:
     return _run_fwht(x, size, None, stagewise=True)
 
 
-def apply_transform(x: torch.Tensor, value: str | TransformSpec, *, rounding: str = "reference") -> torch.Tensor:
+def apply_transform(x: torch.Tensor, value: str | TransformSpec, *, rounding: str = "reference",
+                    amax: torch.Tensor | None = None) -> torch.Tensor:
     """Block-Hadamard along the last axis; a tail shorter than the block passes through.
 
     rounding="reference": round to x.dtype after every stage (bit-equal to the reference
     on bf16/fp16 inputs; no effect for fp32).  rounding="once": fp32 stages, one rounding.
+    amax: optional float32 [1] CUDA tensor that receives max |result| where a kernel runs (a transform
+    that leaves x as it is returns x itself and does not touch it).
     """
     spec = get_transform(value)
     if spec.block_size is None:
@@ -112,7 +119,7 @@ def apply_transform(x: torch.Tensor, value: str | TransformSpec, *, rounding: st
         raise NotImplementedError(f"the FWHT kernel supports block sizes {_SUPPORTED_SIZES}, got {size}")
     dev = x.device if x.is_cuda else torch.device("cuda", torch.cuda.current_device())
     signs = _device_signs(size, spec.seed, dev) if spec.seed is not None else None
-    return _run_fwht(x, size, signs, stagewise=(rounding == "reference"))
+    return _run_fwht(x, size, signs, stagewise=(rounding == "reference"), amax=amax)
 
 
 def hadamard_matrix(size: int, *, device=None, dtype=torch.float32) -> torch.Tensor:
