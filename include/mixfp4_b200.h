@@ -337,6 +337,13 @@ MIXFP4_API int mixfp4_gemm(const void* x, int64_t m, int64_t ldx,
                 int rotation_block, void* y, int out_dtype, int64_t ldy,
                 void* workspace, int64_t workspace_bytes, int* status, int flags, void* stream);
 
+/* mixfp4_gemv_grouped's counterpart for a batch of tokens: up to three stream-layout weights that share x in
+ * one launch, 1 <= M <= 64, x with 16-byte aligned rows (MIXFP4_E_ALIGN otherwise: call mixfp4_gemm per weight).
+ * status as in mixfp4_gemm; flags: MIXFP4_FLAG_OVERLAP_PREVIOUS. */
+MIXFP4_API int mixfp4_gemm_grouped(const void* x, int64_t m, int64_t ldx, int64_t k,
+                        const mixfp4_gemv_segment* segments, int count, int layout, int out_dtype,
+                        int* status, int flags, void* stream);
+
 /* W4A4 in the reference's sense: the activations are rotated (rotation_block 0 or 128; every
  * butterfly stage rounded to bf16, which is what the reference's hook computes on a bf16 tensor,
  * rotation.py:47-58), fake-quantized with mixfp4_fake_quantize(mode = act_mode) and then multiplied

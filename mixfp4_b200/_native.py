@@ -133,6 +133,8 @@ def _declare(h: ctypes.CDLL) -> None:
     h.mixfp4_gemm_workspace_bytes.argtypes = [i64, i64, i64]
     h.mixfp4_gemm.restype = i32
     h.mixfp4_gemm.argtypes = [p, i64, i64, p, p, p, p, i64, i64, i32, p, i32, p, i32, i64, p, i64, p, i32, p]
+    h.mixfp4_gemm_grouped.restype = i32
+    h.mixfp4_gemm_grouped.argtypes = [p, i64, i64, i64, ctypes.POINTER(GemvSegment), i32, i32, i32, p, i32, p]
     h.mixfp4_gemm_a4.restype = i32
     h.mixfp4_gemm_a4.argtypes = [p, i64, i64, p, p, p, p, i64, i64, i32, p, i32, i32, p, i32, i64, p, i64, p, i32, p]
     h.mixfp4_gemm_h128_static_max_bytes.restype = i64
@@ -150,7 +152,7 @@ EXPORTED = (
     "mixfp4_comm_create", "mixfp4_comm_handle_bytes", "mixfp4_comm_handle", "mixfp4_comm_open",
     "mixfp4_comm_buffer_bytes", "mixfp4_comm_buffer", "mixfp4_comm_open_local", "mixfp4_comm_destroy",
     "mixfp4_gemv_allreduce", "mixfp4_set_wait_limit_ns", "mixfp4_check_status",
-    "mixfp4_gemm_workspace_bytes", "mixfp4_gemm", "mixfp4_gemm_a4", "mixfp4_gemm_h128_static_max_bytes", "mixfp4_gemm_h128_static",
+    "mixfp4_gemm_workspace_bytes", "mixfp4_gemm", "mixfp4_gemm_grouped", "mixfp4_gemm_a4", "mixfp4_gemm_h128_static_max_bytes", "mixfp4_gemm_h128_static",
 )
 
 

@@ -42,6 +42,8 @@
 
 #include "common.cuh"
 #include "decode.cuh"
+#include "gemm_small.cuh"
+#include "tcgen05.cuh"
 
 namespace mixfp4 {
 namespace {
@@ -49,8 +51,6 @@ namespace {
 constexpr int BK = 64;                     // K elements per pipeline stage (one 128-byte swizzle row)
 constexpr int kDecodeWarps = 8;             // more transcoder warps were measured: no gain alone, a loss in CTA pairs
 constexpr int kThreads = (3 + kDecodeWarps) * 32;   // x producer, MMA issuer, transcoders, code producer
-constexpr uint64_t kWaitLimitNs = 2000000000ull;   // 2 s: far beyond any legitimate wait
-constexpr uint32_t kMinSpins = 1u << 16;            // ... and at least this many polls
 
 // Tile configuration: kMT sub-tiles of 128 rows of x (each its own TMEM accumulator, all
 // sharing the transcoded weight tile) by kBN weight rows.
@@ -111,137 +111,6 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
     for (int z = 1; z < splits; ++z) sum += partial[((int64_t)z * m + r) * ld_partial + c];
     if (out_dtype == MIXFP4_F32) static_cast<float*>(y)[r * ldy + c] = sum;
     else static_cast<__nv_bfloat16*>(y)[r * ldy + c] = __float2bfloat16_rn(sum);
-}
-
-// ------------------------------------------------------------------------- PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ uint64_t global_timer_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-struct WaitCtx {
-    volatile int* abort_flag;   // shared memory
-    int* status;                // global, may be null
-};
-
-// Bounded wait: false if the limit expired or another thread of the CTA already gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_timer_ns();
-    uint32_t spins = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        if ((++spins & 63u) == 0) {
-            if (*ctx.abort_flag) return false;
-            // both a long time and many polls: a discontinuity of the timer alone never aborts a wait
-            if (spins > kMinSpins && global_timer_ns() - t0 > kWaitLimitNs) {
-                *ctx.abort_flag = 1;
-                if (ctx.status) atomicCAS(ctx.status, 0, code);
-                return false;
-            }
-        }
-    }
-    return true;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
-        : "memory");
-}
-
-// Box of the stream layout's code bytes: coordinates (byte in a row's 64, row in the tile, chunk along K, row tile).
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2,
-                                            int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-
-__device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-
-// D[tmem] (+)= A[smem desc] * B[smem desc], bf16 inputs, fp32 accumulate.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// mbarrier arrive once all previously issued tcgen05.mma of this thread have completed.
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// 32 TMEM lanes x 32 columns of 32-bit: thread i of the warp gets lane base+i, columns c..c+31.
-__device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major bf16 tile with 128-byte swizzle: rows are
-// 128 B apart inside an 8-row group, groups 1024 B apart (stride byte offset), descriptor
-// version 1 (sm_100), layout type 2 (SWIZZLE_128B).  The tile base must be 1024-aligned;
-// a K step of 16 elements advances the start address by 32 B.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
-    const uint64_t lo = ((saddr & 0x3ffffu) >> 4) | (1ull << 16);
-    const uint64_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-    return lo | (hi << 32);
-}
-
-__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ uint4 lds128_lut(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
 }
 
 // Epilogue of one CTA: the transcoder warps read the accumulators from TMEM (lane quarter =
@@ -629,14 +498,6 @@ struct PairCfg {
     static constexpr int kWords = 8 / kThreadsPerRow;                // 4
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // Arrive on the leader CTA's copy of a barrier (from either CTA of the pair).
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & kPeerMask) : "memory");
@@ -916,22 +777,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
 }
 
 // ------------------------------------------------------------------------- host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
-
 // Tensor map of the packed codes; a box is one K step (32 bytes per row) of `box_rows` weight rows.
 // Row-major layouts: the byte matrix [n, kpad/2].  Stream layout: (64 code bytes of a row in a chunk,
 // 16 rows, chunks along K, row tiles), whose box of box_rows/16 tiles lands in shared memory in the
@@ -1125,7 +970,7 @@ extern "C" int64_t mixfp4_gemm_workspace_bytes(int64_t m, int64_t n, int64_t k) 
 static int gemm_run(const void* x, int64_t m, int64_t ldx, const uint8_t* codes, const uint8_t* scales,
                     const uint8_t* fmt, const float* global_scale, int64_t n, int64_t k, int layout, const void* lut,
                     int rotation_block, void* y, int out_dtype, int64_t ldy, void* workspace, int64_t workspace_bytes,
-                    int* status, void* stream, bool x_from_previous_kernel) {
+                    int* status, void* stream, bool x_from_previous_kernel, bool overlap_previous) {
     if (const int rc = check_gemm_args(x, m, ldx, codes, scales, fmt, global_scale, n, k, layout, lut, rotation_block, y,
                                        out_dtype, ldy))
         return rc;
@@ -1148,6 +993,14 @@ static int gemm_run(const void* x, int64_t m, int64_t ldx, const uint8_t* codes,
             MIXFP4_CUDA_CHECK(cudaMemcpy2DAsync(workspace, lda * 2, x, ldx * 2, k * 2, m, cudaMemcpyDeviceToDevice, st));
         }
         xa = workspace;
+    }
+
+    // a few dozen tokens: the decode of the weight is the work (gemm_small.cu; at 48 tokens 15 us against 35 for this
+    // file's tiles on a 4096 x 14336 weight, at 128 20 against 39).  The canonical layout keeps the tiles.
+    if (layout != MIXFP4_LAYOUT_CANONICAL && m <= kSmallMaxTokens) {
+        const mixfp4_gemv_segment seg = {codes, scales, global_scale, lut, y, ldy, n};
+        const bool dependent = rotation_block == 128 || ((x_from_previous_kernel || overlap_previous) && xa == x);
+        return gemm_small(xa, m, lda, k, &seg, 1, layout == MIXFP4_LAYOUT_STREAM, out_dtype, dependent, status, st);
     }
 
     GemmArgs a;
@@ -1194,9 +1047,8 @@ extern "C" int mixfp4_gemm(const void* x, int64_t m, int64_t ldx, const uint8_t*
                            const uint8_t* fmt, const float* global_scale, int64_t n, int64_t k, int layout,
                            const void* lut, int rotation_block, void* y, int out_dtype, int64_t ldy, void* workspace,
                            int64_t workspace_bytes, int* status, int flags, void* stream) {
-    (void)flags;
     return gemm_run(x, m, ldx, codes, scales, fmt, global_scale, n, k, layout, lut, rotation_block, y, out_dtype, ldy,
-                    workspace, workspace_bytes, status, stream, false);
+                    workspace, workspace_bytes, status, stream, false, (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0);
 }
 
 extern "C" int mixfp4_gemm_a4(const void* x, int64_t m, int64_t ldx, const uint8_t* codes, const uint8_t* scales,
@@ -1233,7 +1085,7 @@ extern "C" int mixfp4_gemm_a4(const void* x, int64_t m, int64_t ldx, const uint8
     (void)flags;
     // the quantizer's kernel is the only producer of the staged activations and lets its dependents start early
     return gemm_run(workspace, m, lda, codes, scales, fmt, global_scale, n, k, layout, lut, 0, y, out_dtype, ldy, workspace,
-                    total - kAmaxSlotBytes, status, stream, true);
+                    total - kAmaxSlotBytes, status, stream, true, false);
 }
 
 

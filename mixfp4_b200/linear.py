@@ -19,6 +19,7 @@ from .quant import (HIGH_PRECISION_MODES, PackedWeight, _MODE_CODE, fake_quantiz
                     quantize_packed, quantize_stream, region_shape)
 
 GEMV_MAX_M = 16
+GROUPED_MAX_M = 64       # rows of x that mixfp4_gemm_grouped takes
 _workspaces: dict[tuple, torch.Tensor] = {}
 _status_words: dict[str, torch.Tensor] = {}
 
@@ -156,7 +157,7 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
                                  nat.ptr(packed.fmt), packed.global_scale.data_ptr(), packed.n, packed.k,
                                  packed.layout_code, nat.ptr(packed.lut), fused, y.data_ptr(),
                                  nat.DTYPE_CODE[out_dtype], y.stride(0), nat.ptr(ws), nbytes,
-                                 _status_word(x.device).data_ptr(), 0, stream)
+                                 _status_word(x.device).data_ptr(), nat.gemv_flags(overlap_previous), stream)
             nat.check("mixfp4_gemm", st)
     if bias is not None:
         y += bias.to(y.dtype)
@@ -168,16 +169,16 @@ def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dty
     """[x @ W_i^T for W_i in packs] for weights that take the same x (q/k/v, gate/up).
 
     Decode shapes (at most 16 rows of x), up to three kernel- or stream-layout weights without a folded
-    rotation: one launch (``mixfp4_gemv_grouped``).  Anything else: one ``mixfp4_linear`` per
-    weight, same results.
+    rotation: one launch (``mixfp4_gemv_grouped``); 17 to 64 rows of x and stream-layout weights: one launch
+    too (``mixfp4_gemm_grouped``).  Anything else: one ``mixfp4_linear`` per weight, same results.
     """
     if not packs:
         return []
     k = packs[0].k
     lead = x.shape[:-1]
     m = x.numel() // max(1, x.shape[-1])
-    grouped = (1 <= m <= 16 and 1 <= len(packs) <= 3 and x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] == k
-               and packs[0].layout in ("kernel", "stream")
+    grouped = (1 <= m <= GROUPED_MAX_M and 1 <= len(packs) <= 3 and x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] == k
+               and packs[0].layout in (("kernel", "stream") if m <= GEMV_MAX_M else ("stream",))
                and all(p.k == k and p.layout == packs[0].layout and p.rotation is None for p in packs))
     if grouped:
         out_dtype = x.dtype if out_dtype is None else out_dtype
@@ -191,13 +192,22 @@ def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dty
         for seg, p, y in zip(segs, packs, ys):
             seg.codes, seg.scales, seg.global_scale = p.codes.data_ptr(), nat.ptr(p.scales), p.global_scale.data_ptr()
             seg.lut, seg.y, seg.ldy, seg.n = nat.ptr(p.lut), y.data_ptr(), y.stride(0), p.n
+        flags = nat.gemv_flags(overlap_previous, *[p.lut for p in packs])
         with torch.cuda.device(x.device):
-            st = nat.lib().mixfp4_gemv_grouped(x2.data_ptr(), m, x2.stride(0), k, segs, len(packs),
-                                               packs[0].layout_code, nat.DTYPE_CODE[out_dtype],
-                                               nat.gemv_flags(overlap_previous, *[p.lut for p in packs]),
-                                               nat.stream_ptr(x.device))
+            if m <= GEMV_MAX_M:
+                fn = "mixfp4_gemv_grouped"
+                st = nat.lib().mixfp4_gemv_grouped(x2.data_ptr(), m, x2.stride(0), k, segs, len(packs),
+                                                   packs[0].layout_code, nat.DTYPE_CODE[out_dtype], flags,
+                                                   nat.stream_ptr(x.device))
+            elif x2.data_ptr() % 16 or x2.stride(0) % 8:         # rows that the tensor maps cannot address
+                st = nat.E_SHAPE
+            else:
+                fn = "mixfp4_gemm_grouped"
+                st = nat.lib().mixfp4_gemm_grouped(x2.data_ptr(), m, x2.stride(0), k, segs, len(packs),
+                                                   packs[0].layout_code, nat.DTYPE_CODE[out_dtype],
+                                                   _status_word(x.device).data_ptr(), flags, nat.stream_ptr(x.device))
         if st != nat.E_SHAPE:
-            nat.check("mixfp4_gemv_grouped", st)
+            nat.check(fn, st)
             return [y.reshape(*lead, p.n) for y, p in zip(ys, packs)]
     return [mixfp4_linear(x, p, out_dtype=out_dtype, overlap_previous=overlap_previous and i == 0)
             for i, p in enumerate(packs)]

@@ -1,0 +1,114 @@
+"""The tensor-core kernel for a few dozen tokens (mixfp4_gemm on the stream layout up to 128 rows of x,
+mixfp4_gemm_grouped up to 64) against a float64 product with the dequantized weight.
+
+Tolerance: every MMA adds 16 products to an fp32 accumulator with one rounding or truncation, so a chain of K
+products is off by at most K / 16 units of 2^-23 of its partial sums, which for these zero-mean inputs are of the
+size of the result; a few more for the sums of the chains.  Twice that is allowed."""
+
+import ctypes
+
+import pytest
+import torch
+
+import mixfp4_b200 as mx
+from mixfp4_b200 import _native as nat
+from mixfp4_b200 import synth
+
+
+def tolerance(k: int) -> float:
+    return 2 * (k / 16 + 8) * 2.0 ** -23
+
+
+def weight(n, k, seed):
+    w = synth.student_t_weight(n, k, seed).cuda()
+    packed = mx.quantize_packed(w)[0].to_stream_layout()
+    return packed, packed.dequantize().double()
+
+
+def check(y, x, wd, k, out):
+    ref = x.double() @ wd.T
+    rel = ((y.double() - ref).norm() / ref.norm()).item()
+    assert rel <= tolerance(k) + (2.0 ** -9 if out == torch.bfloat16 else 0.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 96, 127, 128])
+@pytest.mark.parametrize("n,k", [(16, 16), (17, 128), (130, 96), (128, 256), (1000, 1112), (4240, 640), (2048, 4096), (19000, 384)])
+def test_against_float64(m, n, k):
+    packed, wd = weight(n, k, n + k)
+    x = synth.activations(m, k, m).cuda()
+    for out in (torch.float32, torch.bfloat16):
+        y = mx.mixfp4_linear(x, packed, out_dtype=out)
+        check(y, x, wd, k, out)
+    wide = torch.zeros((m, k + 3), dtype=torch.bfloat16, device="cuda")     # rows that a tensor map cannot address
+    wide[:, 1:k + 1] = x
+    assert torch.equal(mx.mixfp4_linear(wide[:, 1:k + 1], packed), mx.mixfp4_linear(x, packed))
+    bare = mx.PackedWeight(packed.codes, packed.scales, None, packed.global_scale, n, k, None, "stream", None)
+    assert torch.equal(mx.mixfp4_linear(x, bare), mx.mixfp4_linear(x, packed))       # the kernel builds the decode table
+    assert torch.equal(mx.mixfp4_linear(x, packed.to_canonical().to_kernel_layout()), mx.mixfp4_linear(x, packed))
+    assert mx.gemm_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [17, 48, 64])
+@pytest.mark.parametrize("ns,k", [((256, 64, 64), 512), ((4096, 1024, 1000), 4096), ((300, 17), 1112), ((14336, 14336), 640)])
+def test_grouped_repeats_and_matches(m, ns, k):
+    """One launch for weights that share x, chained to the launch before; thirty launches in a row give the same bits
+    (the stages of the weight ring are reused hundreds of times: a release that came too early shows here)."""
+    ws = [weight(n, k, i + k) for i, n in enumerate(ns)]
+    packs = [p for p, _ in ws]
+    x = synth.activations(m, k, m).cuda()
+    first = mx.mixfp4_linear_grouped(x, packs, out_dtype=torch.float32)
+    for y, (_, wd) in zip(first, ws):
+        check(y, x, wd, k, torch.float32)
+    runs = [mx.mixfp4_linear_grouped(x, packs, out_dtype=torch.float32, overlap_previous=True) for _ in range(30)]
+    assert all(torch.equal(a, b) for run in runs for a, b in zip(run, first))
+    assert mx.gemm_status() == 0
+
+
+@pytest.mark.gpu
+def test_chain_under_dependent_launches_and_graph():
+    """Each launch reads the one before it; overlapped launches in a graph give the bits of separate ones."""
+    up, _ = weight(2048, 1024, 1)
+    down, _ = weight(1024, 2048, 2)
+    x = synth.activations(40, 1024, 3).cuda()
+
+    def run(overlap):
+        h = x
+        for _ in range(4):
+            h = mx.mixfp4_linear(mx.mixfp4_linear(h, up, overlap_previous=overlap), down, overlap_previous=overlap)
+            h = h / h.float().abs().max().to(h.dtype)
+        return h
+    want = run(False)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        run(True)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = run(True)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+
+
+def test_grouped_entry_checks_its_arguments():
+    lib = nat.lib()
+    one = ctypes.c_void_p(16)
+    seg = (nat.GemvSegment * 1)()
+    seg[0].codes, seg[0].global_scale, seg[0].y, seg[0].ldy, seg[0].n = 16, 16, 16, 64, 64
+    call = lambda x=one, m=17, ldx=64, k=64, s=seg, count=1, layout=nat.LAYOUT_STREAM, out=nat.F32: lib.mixfp4_gemm_grouped(
+        x, m, ldx, k, s, count, layout, out, None, 0, None)
+    assert call(layout=nat.LAYOUT_KERNEL) == nat.E_MODE
+    assert call(x=None) == nat.E_NULL and call(s=None) == nat.E_NULL
+    assert call(m=0) == nat.E_SHAPE and call(m=65) == nat.E_SHAPE and call(count=4) == nat.E_SHAPE and call(ldx=63) == nat.E_SHAPE
+    assert call(out=nat.F16) == nat.E_DTYPE
+    assert call(x=ctypes.c_void_p(8)) == nat.E_ALIGN and call(ldx=68) == nat.E_ALIGN
+    seg[0].ldy = 63
+    assert call() == nat.E_SHAPE
+    seg[0].ldy, seg[0].codes = 64, 8
+    assert call() == nat.E_ALIGN
+    seg[0].codes, seg[0].y = 16, None
+    assert call() == nat.E_NULL
