@@ -1,5 +1,5 @@
 // Dequant-linear for a server's batch of tokens (more than the matrix-vector kernels take, up to 128 rows of
-// x) on the stream or the kernel layout of the packed weight:
+// x; also fewer whose x is too large for those kernels' shared memory) on the stream or the kernel layout of the packed weight:
 //   y[M,N] = x[M,K] * W[N,K]^T, replacing F.linear on the dequantized weight (project_quant/modeling.py:629).
 //
 // At these sizes every weight is decoded once and used for a few dozen tokens, so the work is the decode, not
@@ -78,6 +78,7 @@ struct SmallArgs {
     uint32_t inv_cluster, inv_units;                // 2^16 / cluster (rounded up), 2^32 / units (rounded down)
     int d_cols;                                     // TMEM columns of an accumulator: np rounded up to 32
     int chains;                                     // accumulators per piece (1, 2 or 4), units in turn: see gemm_small
+    int flush;                                      // 0, or units after which a piece's accumulators are added up in registers
     int a_stages;                                   // A stages (units, with their x): 4, or 2 when the accumulators need the columns
     int x_pair;                                     // x comes in boxes of 2 x 64 K (K a multiple of 64), else one by one
     int w_stages, lut_shift;                        // weight stages (a power of two); 2^lut_shift copies of the decode table
@@ -92,14 +93,15 @@ __device__ __forceinline__ int tile_row(int q, int lane) { return (4 * (q >> 1) 
 
 // shared-memory map (offsets from a 1024-aligned base)
 struct SmallLayout {
-    uint32_t x, codes, lut, bars, misc, bytes;
+    uint32_t x, codes, lut, parts, bars, misc, bytes;
 };
-__host__ __device__ inline SmallLayout small_layout(int np, int nseg, int w_stages, int a_stages, int lut_shift) {
+__host__ __device__ inline SmallLayout small_layout(int np, int nseg, int w_stages, int a_stages, int lut_shift, int flush) {
     SmallLayout l;
     l.x = 0;
     l.codes = l.x + (uint32_t)a_stages * np * 256;
     l.lut = l.codes + (uint32_t)w_stages * kUnitBytes;
-    l.bars = l.lut + (uint32_t)nseg * (4096u << lut_shift);
+    l.parts = l.lut + (uint32_t)nseg * (4096u << lut_shift);
+    l.bars = l.parts + (flush ? (uint32_t)np * kTileRows * 8u : 0u);          // sums of cut tiles; without flushes the rings take them
     l.misc = l.bars + (2 * kMaxWStages + 2 * kUnitStages + 6) * 8;
     l.bytes = l.misc + 16 + 16 + 1024;                   // + alignment slack
     return l;
@@ -200,7 +202,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;            // the same offset in every CTA of the cluster
     uint8_t* gen = smem_raw + (base - raw);
-    const SmallLayout L = small_layout(a.np, a.nseg, a.w_stages, a.a_stages, a.lut_shift);
+    const SmallLayout L = small_layout(a.np, a.nseg, a.w_stages, a.a_stages, a.lut_shift, a.flush);
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // provably warp-uniform
     const int S = a.units, np = a.np;
@@ -374,7 +376,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         const uint32_t box16 = (uint32_t)np * 128u >> 4;                   // 64 K of x, in descriptor units
         const uint64_t x_desc0 = make_smem_desc(base + L.x);
         uint32_t d_set = tmem_base;
-        int piece = 0, done = 0, left = min(S - sub_first, cnt);    // units of the piece done and left
+        int piece = 0, done = 0, left = min(S - sub_first, cnt);    // units of the piece done (since the last flush) and left
+        int set = 0, set_par = 1;                                   // flushing: sets in turn
         bool ok = true;
         for (int u = 0; u < cnt; ++u) {
             ok = warp_wait(full_a(u & 3), (u >> 2) & 1, ctx, 4);
@@ -389,7 +392,17 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                 umma_ts_bf16_if(lead, d_tmem, a_tmem + k * 8, db + (k >> 2) * box16 + 2u * (k & 3), idesc, k == 0 ? accumulate : 1u);
             umma_commit_if(lead, empty_a(u & 3));
             ++done;
-            if (--left == 0) {                                      // the piece is complete; the next one's accumulators
+            --left;
+            if (a.flush) {
+                if (left == 0 || done == a.flush) {
+                    umma_commit_if(lead, full_d(set));
+                    if (left == 0) left = min(S, cnt - (u + 1));
+                    done = 0;
+                    if (++set == 3) { set = 0; set_par ^= 1; }
+                    d_set = tmem_base + (uint32_t)(set * a.chains) * d_cols;
+                    if (u + 1 < cnt && !warp_wait(empty_d(set), set_par, ctx, 10)) break;
+                }
+            } else if (left == 0) {                                   // the piece is complete; the next one's accumulators
                 umma_commit_if(lead, full_d(d_of(piece)));
                 ++piece;
                 left = min(S, cnt - (u + 1));
@@ -412,7 +425,45 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     } else if (warp >= 4 && warp < 8) {
         // epilogue of the tiles this run holds from end to end
         const int q = warp & 3, row = tile_row(q, lane);
-        for (int p = 0; p < npieces; ++p) {
+        int set = 0, par = 0;
+        for (int p = 0; a.flush && p < npieces; ++p) {              // 16 tokens at most: the sums fit in registers
+            float sum[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum[j] = 0.0f;
+            const int lo = (tile_first + p) * S;
+            int len = min(lo + S, ub) - max(lo, ua);
+            bool ok = true;
+            for (; len > 0 && ok; len -= a.flush) {
+                ok = warp_wait(full_d(set), par, ctx, 6);
+                if (!ok) break;
+                tcgen05_fence_after();
+                for (int i = 0; i < min(a.chains, len); ++i) {
+                    float v[16];
+                    tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(set * a.chains + i) * d_cols, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sum[j] += v[j];
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty_d(set));
+                if (++set == 3) { set = 0; par ^= 1; }
+            }
+            if (!ok) break;
+            if (piece_whole(p)) {
+                const int tile = t0 + tile_first + p, sg = seg_of(tile);
+                const SmallSegment& seg = a.seg[sg];
+                const int n0 = (tile - seg_first(sg)) * kTileRows + row;
+                if (n0 < seg.n)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (j < a.m) store_y(seg, a.out_dtype, j, n0, sum[j]);
+            } else {
+                float* part = reinterpret_cast<float*>(gen + L.parts) + (p == 0 ? 0 : np * kTileRows) + q * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) part[j * kTileRows] = sum[j];
+            }
+        }
+        for (int p = 0; !a.flush && p < npieces; ++p) {
             const int d = d_of(p);
             if (!warp_wait(full_d(d), p == 0 ? 0 : ((p - 1) >> 1) & 1, ctx, 6)) break;
             if (!piece_whole(p)) continue;
@@ -503,11 +554,13 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     if (a.cluster > 1) {
         // Tiles cut by run boundaries.  All copies have landed and all MMAs are done (the epilogue warps have waited
         // for every piece), so the rings are free: [first piece, last piece][token][TMEM lane] fp32.
-        float* parts = reinterpret_cast<float*>(gen);
+        // (Flushed sums are there already, in their own place.)
+        const uint32_t parts_at = a.flush ? L.parts : 0u;
+        float* parts = reinterpret_cast<float*>(gen + parts_at);
         const uint32_t part_stride = (uint32_t)np * kTileRows;
         const int tl_index = (warp & 3) * 32 + lane;
         __syncthreads();
-        if (warp >= 4 && warp < 8) {
+        if (!a.flush && warp >= 4 && warp < 8) {
             tcgen05_fence_after();
             for (int i = 0; i < 2; ++i) {
                 const int p = i == 0 ? 0 : npieces - 1;
@@ -534,7 +587,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
 #pragma unroll
             for (int w2 = 0; w2 < kMaxCluster; ++w2)
                 if (w2 < share)
-                    src[w2] = peer_addr(base + (uint32_t)lane * 16u + (w2 == 0 && (packed >> 16) ? part_stride * 4u : 0u), (uint32_t)(wf + w2));
+                    src[w2] = peer_addr(base + parts_at + (uint32_t)lane * 16u + (w2 == 0 && (packed >> 16) ? part_stride * 4u : 0u), (uint32_t)(wf + w2));
             for (int b = (rank - wf) + share * warp; b < a.m; b += share * (kThreadsS / 32)) {
                 float4 v[kMaxCluster];
 #pragma unroll
@@ -699,17 +752,20 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
     // fp64), so a piece's units go to as many accumulators in turn as there is room for and the sums are added in fp32.
     a.d_cols = (a.np + 31) / 32 * 32;
     a.chains = a.d_cols <= 32 ? 4 : a.d_cols <= 64 ? 2 : 1;
+    // Up to 16 tokens stand in for matrix-vector kernels that split K finely: chains of 256 products at most, added up in
+    // the epilogue warps' registers.
+    a.flush = a.np == 16 ? 2 * a.chains : 0;
     a.a_stages = 3 * a.chains * a.d_cols + 4 * 64 <= (int)kTmemColsS ? 4 : 2;
     // shared memory: eight weight stages and eight copies of the tables where they fit
     const int choices[6][2] = {{8, 3}, {8, 2}, {4, 3}, {4, 2}, {4, 1}, {4, 0}};
     for (const auto& c : choices) {
         a.w_stages = c[0];
         a.lut_shift = c[1];
-        if (small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift).bytes <= kSmemLimitS) break;
+        if (small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.flush).bytes <= kSmemLimitS) break;
     }
-    const SmallLayout L = small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift);
+    const SmallLayout L = small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.flush);
     // (the partial sums of cut tiles, 2 * np * 512 bytes, go where the rings were)
-    if (L.bytes > kSmemLimitS || (uint32_t)a.np * kTileRows * 8u > L.lut) return MIXFP4_E_SHAPE;
+    if (L.bytes > kSmemLimitS || (!a.flush && (uint32_t)a.np * kTileRows * 8u > L.lut)) return MIXFP4_E_SHAPE;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(plan.cluster * plan.nclusters));
     cfg.blockDim = dim3(kThreadsS);

@@ -33,6 +33,7 @@
 // 4-bit codes (one 32-bit word) become four bf16x2 registers with byte permutes
 // (decode.cuh).  The accumulation is the tensor core's fp32.
 
+#include "gemm_small.cuh"
 #include "gemv_common.cuh"
 
 namespace mixfp4 {
@@ -695,7 +696,15 @@ extern "C" int mixfp4_gemv(const void* x, int64_t m, int64_t ldx, const uint8_t*
     if (streamed) {
         const mixfp4_gemv_segment seg = {codes, nullptr, global_scale, lut, y, ldy, n};
         const int rc = gemv_stream(x, m, ldx, k, &seg, 1, out_dtype, flags, nullptr, nullptr, st);
-        if (rc != MIXFP4_E_SHAPE) return rc;     // x too large for shared memory: the kernel below stages it
+        if (rc != MIXFP4_E_SHAPE) return rc;
+        // x too large for shared memory: the tensor-core kernel streams it beside the weight (4096 x 14336, 12 tokens:
+        // 33.6 -> 16.4 us); rows that a tensor map cannot address are staged by the kernel below
+        if (aligned(x, 16) && ldx % 8 == 0) {
+            int* status = nullptr;
+            if (const int rs = stream_status_word(&status)) return rs;
+            const int rg = gemm_small(x, m, ldx, k, &seg, 1, true, out_dtype, (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0, status, st);
+            if (rg != MIXFP4_E_SHAPE) return rg;
+        }
     }
     GemvArgs a;
     a.x = static_cast<const __nv_bfloat16*>(x);

@@ -121,4 +121,7 @@ int gemv_stream(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_g
 // Limit of the bounded device-side waits (2 s unless mixfp4_set_wait_limit_ns changed it).
 uint64_t wait_limit_ns();
 
+// gemv_stream.cu: the current device's status word of the decode kernels.
+int stream_status_word(int** out);
+
 }  // namespace mixfp4

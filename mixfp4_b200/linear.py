@@ -194,14 +194,15 @@ def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dty
             seg.lut, seg.y, seg.ldy, seg.n = nat.ptr(p.lut), y.data_ptr(), y.stride(0), p.n
         flags = nat.gemv_flags(overlap_previous, *[p.lut for p in packs])
         with torch.cuda.device(x.device):
+            tma_rows = x2.data_ptr() % 16 == 0 and x2.stride(0) % 8 == 0        # a tensor map can address them
             if m <= GEMV_MAX_M:
                 fn = "mixfp4_gemv_grouped"
                 st = nat.lib().mixfp4_gemv_grouped(x2.data_ptr(), m, x2.stride(0), k, segs, len(packs),
                                                    packs[0].layout_code, nat.DTYPE_CODE[out_dtype], flags,
                                                    nat.stream_ptr(x.device))
-            elif x2.data_ptr() % 16 or x2.stride(0) % 8:         # rows that the tensor maps cannot address
-                st = nat.E_SHAPE
             else:
+                st = nat.E_SHAPE
+            if st == nat.E_SHAPE and packs[0].layout == "stream" and tma_rows:   # too many rows, or too large to stay resident
                 fn = "mixfp4_gemm_grouped"
                 st = nat.lib().mixfp4_gemm_grouped(x2.data_ptr(), m, x2.stride(0), k, segs, len(packs),
                                                    packs[0].layout_code, nat.DTYPE_CODE[out_dtype],

@@ -67,6 +67,24 @@ def test_grouped_repeats_and_matches(m, ns, k):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,ns,k", [(8, (200,), 14336), (9, (4096,), 14336), (16, (4096,), 14336), (12, (3000, 3000), 8192),
+                                    (16, (128, 100, 16), 9000), (13, (28672,), 8192)])
+def test_few_tokens_with_a_large_x(m, ns, k):
+    """Up to 16 rows of x that do not fit in the matrix-vector kernel's shared memory: chains of at most 256 products,
+    so the error stays at that of the matrix-vector kernels."""
+    ws = [weight(n, k, n + k) for n in ns]
+    x = synth.activations(m, k, m).cuda()
+    ys = mx.mixfp4_linear_grouped(x, [p for p, _ in ws], out_dtype=torch.float32)
+    for y, (p, wd) in zip(ys, ws):
+        ref = x.double() @ wd.T
+        assert ((y.double() - ref).norm() / ref.norm()).item() <= tolerance(256)
+        assert torch.equal(mx.mixfp4_linear(x, p).float(), mx.mixfp4_linear(x, p).float())
+    runs = [mx.mixfp4_linear_grouped(x, [p for p, _ in ws], out_dtype=torch.float32, overlap_previous=True) for _ in range(10)]
+    assert all(torch.equal(a, b) for run in runs for a, b in zip(run, ys))
+    assert mx.gemm_status() == 0 and mx.decode_status() == 0
+
+
+@pytest.mark.gpu
 def test_chain_under_dependent_launches_and_graph():
     """Each launch reads the one before it; overlapped launches in a graph give the bits of separate ones."""
     up, _ = weight(2048, 1024, 1)
