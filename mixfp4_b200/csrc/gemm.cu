@@ -1000,7 +1000,8 @@ static int gemm_run(const void* x, int64_t m, int64_t ldx, const uint8_t* codes,
     if (layout != MIXFP4_LAYOUT_CANONICAL && m <= kSmallMaxTokens) {
         const mixfp4_gemv_segment seg = {codes, scales, global_scale, lut, y, ldy, n};
         const bool dependent = rotation_block == 128 || ((x_from_previous_kernel || overlap_previous) && xa == x);
-        return gemm_small(xa, m, lda, k, &seg, 1, layout == MIXFP4_LAYOUT_STREAM, out_dtype, dependent, status, st);
+        const int rc = gemm_small(xa, m, lda, k, &seg, 1, layout == MIXFP4_LAYOUT_STREAM, out_dtype, dependent, status, st);
+        if (rc != MIXFP4_E_SHAPE) return rc;         // sizes beyond its index range: the tiles below
     }
 
     GemmArgs a;

@@ -31,7 +31,7 @@
 //
 // The single-warp roles set the pace unless they are lean: measured on gate + up (28672 x 4096, 48 tokens), integer
 // divisions in their loops 66 us whatever the decode did, running counters 39 us, one barrier, one box and
-// predicated (not branched) issue per unit 30 to 34 us.
+// predicated (not branched) issue per unit 30 us, two more A stages 28 us.
 
 #include <string.h>
 
@@ -78,7 +78,9 @@ struct SmallArgs {
     uint32_t inv_cluster, inv_units;                // 2^16 / cluster (rounded up), 2^32 / units (rounded down)
     int d_cols;                                     // TMEM columns of an accumulator: np rounded up to 32
     int chains;                                     // accumulators per piece (1, 2 or 4), units in turn: see gemm_small
+    int slots;                                      // sums of cut tiles kept apart from the rings: 0, 1 or 2
     int flush;                                      // 0, or units after which a piece's accumulators are added up in registers
+    int sets;                                       // sets of accumulators: 3, or 2 when no piece has to stay in TMEM
     int a_stages;                                   // A stages (units, with their x): 4, or 2 when the accumulators need the columns
     int x_pair;                                     // x comes in boxes of 2 x 64 K (K a multiple of 64), else one by one
     int w_stages, lut_shift;                        // weight stages (a power of two); 2^lut_shift copies of the decode table
@@ -95,13 +97,13 @@ __device__ __forceinline__ int tile_row(int q, int lane) { return (4 * (q >> 1) 
 struct SmallLayout {
     uint32_t x, codes, lut, parts, bars, misc, bytes;
 };
-__host__ __device__ inline SmallLayout small_layout(int np, int nseg, int w_stages, int a_stages, int lut_shift, int flush) {
+__host__ __device__ inline SmallLayout small_layout(int np, int nseg, int w_stages, int a_stages, int lut_shift, int slots) {
     SmallLayout l;
     l.x = 0;
     l.codes = l.x + (uint32_t)a_stages * np * 256;
     l.lut = l.codes + (uint32_t)w_stages * kUnitBytes;
     l.parts = l.lut + (uint32_t)nseg * (4096u << lut_shift);
-    l.bars = l.parts + (flush ? (uint32_t)np * kTileRows * 8u : 0u);          // sums of cut tiles; without flushes the rings take them
+    l.bars = l.parts + (uint32_t)slots * np * kTileRows * 4u;                  // sums of cut tiles; without slots the rings take them
     l.misc = l.bars + (2 * kMaxWStages + 2 * kUnitStages + 6) * 8;
     l.bytes = l.misc + 16 + 16 + 1024;                   // + alignment slack
     return l;
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;            // the same offset in every CTA of the cluster
     uint8_t* gen = smem_raw + (base - raw);
-    const SmallLayout L = small_layout(a.np, a.nseg, a.w_stages, a.a_stages, a.lut_shift, a.flush);
+    const SmallLayout L = small_layout(a.np, a.nseg, a.w_stages, a.a_stages, a.lut_shift, a.slots);
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // provably warp-uniform
     const int S = a.units, np = a.np;
@@ -307,9 +309,11 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     tcgen05_fence_after();
     const uint32_t tmem_base = warp < 2 ? 0u : __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t d_cols = (uint32_t)a.d_cols;               // TMEM: three sets of accumulators | A stages
-    const uint32_t a_base = tmem_base + 3 * a.chains * d_cols;
-    // accumulator set of a run's piece p: the first piece may be a cut tile that has to stay
-    auto d_of = [&](int p) { return p == 0 ? 0 : 1 + ((p - 1) & 1); };
+    const uint32_t a_base = tmem_base + a.sets * a.chains * d_cols;
+    // accumulator set of a run's piece p and how often it has been used before: two sets in turn, or three, where the
+    // first piece may be a cut tile that has to stay in its own
+    auto d_of = [&](int p) { return a.sets == 2 ? p & 1 : p == 0 ? 0 : 1 + ((p - 1) & 1); };
+    auto d_use = [&](int p) { return a.sets == 2 ? p >> 1 : p == 0 ? 0 : (p - 1) >> 1; };
     const int npieces = div_units(ub - 1) - tile_first + 1;
     auto piece_whole = [&](int p) {
         const int tile = tile_first + p;
@@ -398,7 +402,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                     umma_commit_if(lead, full_d(set));
                     if (left == 0) left = min(S, cnt - (u + 1));
                     done = 0;
-                    if (++set == 3) { set = 0; set_par ^= 1; }
+                    if (++set == a.sets) { set = 0; set_par ^= 1; }
                     d_set = tmem_base + (uint32_t)(set * a.chains) * d_cols;
                     if (u + 1 < cnt && !warp_wait(empty_d(set), set_par, ctx, 10)) break;
                 }
@@ -408,8 +412,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                 left = min(S, cnt - (u + 1));
                 done = 0;
                 d_set = tmem_base + (uint32_t)(d_of(piece) * a.chains) * d_cols;
-                // sets 1 and 2 are used by every second piece; set 0 once
-                if (piece >= 3 && left > 0 && !warp_wait(empty_d(d_of(piece)), (((piece - 1) >> 1) & 1) ^ 1, ctx, 10)) break;
+                if (d_use(piece) > 0 && left > 0 && !warp_wait(empty_d(d_of(piece)), (d_use(piece) & 1) ^ 1, ctx, 10)) break;
             }
         }
     } else if (warp == 3) {
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty_d(set));
-                if (++set == 3) { set = 0; par ^= 1; }
+                if (++set == a.sets) { set = 0; par ^= 1; }
             }
             if (!ok) break;
             if (piece_whole(p)) {
@@ -465,8 +468,9 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         }
         for (int p = 0; !a.flush && p < npieces; ++p) {
             const int d = d_of(p);
-            if (!warp_wait(full_d(d), p == 0 ? 0 : ((p - 1) >> 1) & 1, ctx, 6)) break;
-            if (!piece_whole(p)) continue;
+            if (!warp_wait(full_d(d), d_use(p) & 1, ctx, 6)) break;
+            const bool whole = piece_whole(p);
+            if (!whole && a.slots == 0) continue;                   // stays in TMEM to the end
             tcgen05_fence_after();
             const int tile = t0 + tile_first + p, sg = seg_of(tile);
             const SmallSegment& seg = a.seg[sg];
@@ -474,10 +478,15 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
             for (int c = 0; c < np; c += 16) {
                 float v[16];
                 load_piece(p, c, v);
-                if (n0 < seg.n)
+                if (!whole) {                                       // a cluster of two: one cut tile per run
+                    float* part = reinterpret_cast<float*>(gen + L.parts) + c * kTileRows + q * 32 + lane;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) part[j * kTileRows] = v[j];
+                } else if (n0 < seg.n) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
                         if (c + j < a.m) store_y(seg, a.out_dtype, c + j, n0, v[j]);
+                }
             }
             tcgen05_fence_before();
             __syncwarp();
@@ -554,13 +563,13 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     if (a.cluster > 1) {
         // Tiles cut by run boundaries.  All copies have landed and all MMAs are done (the epilogue warps have waited
         // for every piece), so the rings are free: [first piece, last piece][token][TMEM lane] fp32.
-        // (Flushed sums are there already, in their own place.)
-        const uint32_t parts_at = a.flush ? L.parts : 0u;
+        // (Sums that have slots are there already.)
+        const uint32_t parts_at = a.slots ? L.parts : 0u;
         float* parts = reinterpret_cast<float*>(gen + parts_at);
         const uint32_t part_stride = (uint32_t)np * kTileRows;
         const int tl_index = (warp & 3) * 32 + lane;
         __syncthreads();
-        if (!a.flush && warp >= 4 && warp < 8) {
+        if (a.slots == 0 && warp >= 4 && warp < 8) {
             tcgen05_fence_after();
             for (int i = 0; i < 2; ++i) {
                 const int p = i == 0 ? 0 : npieces - 1;
@@ -587,7 +596,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
 #pragma unroll
             for (int w2 = 0; w2 < kMaxCluster; ++w2)
                 if (w2 < share)
-                    src[w2] = peer_addr(base + parts_at + (uint32_t)lane * 16u + (w2 == 0 && (packed >> 16) ? part_stride * 4u : 0u), (uint32_t)(wf + w2));
+                    src[w2] = peer_addr(base + parts_at + (uint32_t)lane * 16u + (w2 == 0 && (packed >> 16) && a.slots != 1 ? part_stride * 4u : 0u), (uint32_t)(wf + w2));
             for (int b = (rank - wf) + share * warp; b < a.m; b += share * (kThreadsS / 32)) {
                 float4 v[kMaxCluster];
 #pragma unroll
@@ -659,20 +668,22 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
 
 }  // namespace
 
-// Work split: the cluster size with the shortest longest run; an exchange of partial sums costs about as much as
-// three units (about 0.35 us each) plus a little per CTA.  One decode step of 48 tokens through the linears of eight
-// 8B-shaped decoder layers: 1358 us with the 128-row tiles of gemm_kernel (seven launches and up to seven split-K sums
-// a layer), 652 us with four launches of this kernel.  Launches alone, 48 tokens: 4096 x 4096 9.3 us, 6144 x 4096 in
-// three weights 11.9 us, 28672 x 4096 in two 38.7 us, 4096 x 14336 17.2 us; the decode's byte permutes keep the ALU
-// busy for 476 of the 620 to 700 cycles a unit takes.
+// Work split: the cluster size with the shortest longest run.  In units (about 0.37 us each), an exchange of partial
+// sums costs next to nothing between two CTAs and about nine units among four or more; odd sizes lose SMs and start
+// late (28672 x 4096, 48 tokens: 30.5, 30.3, 37.7, 31.4, 32.7, 31.6, 36.4, 33.0 us for 1 to 8 CTAs; 4096 x 14336: 44.5,
+// 24.3, 19.9, 17.4, 22.8, 18.0, 22.5, 20.4 us), and are left out.
+// One decode step of 48 tokens through the linears of eight 8B-shaped decoder layers: 1358 us with the 128-row tiles of
+// gemm_kernel (seven launches and up to seven split-K sums a layer), 508 us with four launches of this kernel.  Launches
+// alone, 48 tokens: 4096 x 4096 8.7 us, 6144 x 4096 in three weights 10.6 us, 28672 x 4096 in two 27.9 us, 4096 x 14336
+// 17.3 us.  The decode's byte permutes keep the ALU busy for 476 cycles of a unit.
 SmallPlan plan_small(int ntiles, int units, const int* clusters) {
     SmallPlan best = {0, 0};
     double t_best = 1e300;
-    for (int c = 1; c <= kMaxCluster && c <= units; ++c) {
+    for (int c = 1; c <= kMaxCluster && c <= units; c += c == 1 ? 1 : 2) {
         if (clusters[c] < 1) continue;
         const int n = ntiles < clusters[c] ? ntiles : clusters[c];
         const int64_t longest = ((int64_t)((ntiles + n - 1) / n) * units + c - 1) / c;
-        const double t = (double)longest + (c > 1 ? 3.0 + 0.25 * c : 0.0);
+        const double t = (double)longest + (c == 1 ? 0.0 : c == 2 ? 1.0 : 9.0);
         if (t < t_best) { t_best = t; best.cluster = c; best.nclusters = n; }
     }
     return best;
@@ -747,7 +758,7 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
     a.split_more = RunSplit{n1 / a.cluster, n1 % a.cluster};
     a.inv_cluster = 65536u / (uint32_t)a.cluster + 1;
     a.inv_units = a.units == 1 ? 0xffffffffu : (uint32_t)((1ull << 32) / (uint32_t)a.units);
-    // TMEM (512 columns): three sets of accumulators, 4 or 2 A stages of 64 columns.  The tensor core's accumulation
+    // TMEM (512 columns): two or three sets of accumulators, 4 or 2 A stages of 64 columns.  The tensor core's accumulation
     // error grows with the number of products in a chain (3.7e-6 of the result after 4096, 8e-7 after 1024, against
     // fp64), so a piece's units go to as many accumulators in turn as there is room for and the sums are added in fp32.
     a.d_cols = (a.np + 31) / 32 * 32;
@@ -755,17 +766,22 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
     // Up to 16 tokens stand in for matrix-vector kernels that split K finely: chains of 256 products at most, added up in
     // the epilogue warps' registers.
     a.flush = a.np == 16 ? 2 * a.chains : 0;
-    a.a_stages = 3 * a.chains * a.d_cols + 4 * 64 <= (int)kTmemColsS ? 4 : 2;
+    // A run has a cut tile at each end at most, in a cluster of two only at one; sums that leave TMEM as soon as their
+    // piece is complete free a set of accumulators for two more A stages (28672 x 4096, 48 tokens: about a tenth).
+    // (Beyond 64 tokens shared memory has no room for them.)
+    a.slots = a.cluster == 1 || a.np > 64 ? 0 : a.flush ? 2 : a.cluster == 2 ? 1 : 0;
+    a.sets = a.np <= 64 && (a.cluster <= 2 || a.flush) ? 2 : 3;
+    a.a_stages = a.sets * a.chains * a.d_cols + 4 * 64 <= (int)kTmemColsS ? 4 : 2;
     // shared memory: eight weight stages and eight copies of the tables where they fit
     const int choices[6][2] = {{8, 3}, {8, 2}, {4, 3}, {4, 2}, {4, 1}, {4, 0}};
     for (const auto& c : choices) {
         a.w_stages = c[0];
         a.lut_shift = c[1];
-        if (small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.flush).bytes <= kSmemLimitS) break;
+        if (small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.slots).bytes <= kSmemLimitS) break;
     }
-    const SmallLayout L = small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.flush);
+    const SmallLayout L = small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.slots);
     // (the partial sums of cut tiles, 2 * np * 512 bytes, go where the rings were)
-    if (L.bytes > kSmemLimitS || (!a.flush && (uint32_t)a.np * kTileRows * 8u > L.lut)) return MIXFP4_E_SHAPE;
+    if (L.bytes > kSmemLimitS || (a.slots == 0 && (uint32_t)a.np * kTileRows * 8u > L.lut)) return MIXFP4_E_SHAPE;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(plan.cluster * plan.nclusters));
     cfg.blockDim = dim3(kThreadsS);
