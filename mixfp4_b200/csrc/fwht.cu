@@ -249,12 +249,21 @@ __global__ void __launch_bounds__(kFastThreads) fwht128_kernel(const T* __restri
 // single one of the packed add / fma.  Layout as in fwht128_kernel (a pair of lanes per block, chunks h, h+2,
 // ... per lane), values kept as words of two neighbouring elements: stride 1 pairs the halves of a word
 // ((l, l) + (r, r) * (1, -1) in one fma), strides 2 and 4 pair words of a chunk, stride 8 the neighbouring
-// lane's word, strides 16 to 64 the chunks.  The final division is the fp32 one of fwht128_kernel, rounded
-// once more to the input type.  amax (optional): the largest output magnitude, for the activation
+// lane's word, strides 16 to 64 the chunks.  The final division, in fp32 and rounded once more to the input type, is
+// one multiplication by the fp32 number just above 1 / sqrt(128): after the second rounding it gives the quotient's
+// bits for every 16-bit pattern of either type (mixfp4_selftest_division sweeps all of them), zeros, subnormals and
+// infinities included.  (The exact fp32 quotient took a range check per lane, and sums of 16-bit values are exactly
+// zero so often that nearly every warp went through its division-by-division branch: 1467 instructions a warp.
+// Loading a rotated 14336 x 4096 projection: 169 -> 127 us.)  amax (optional): the largest output magnitude, for the activation
 // quantizer that follows (one atomic maximum per CTA on the float's bit pattern).
+// The factor that stands for the division (see above).
+__device__ __forceinline__ float quotient_factor(float root) { return __uint_as_float(__float_as_uint(__frcp_rn(root)) + 1u); }
+
 template <typename T> struct Pair;
 template <> struct Pair<__nv_bfloat16> {
     using type = __nv_bfloat162;
+    __device__ static type abs2(type v) { return __habs2(v); }
+    __device__ static type max2(type a, type b) { return __hmax2(a, b); }
     __device__ static type make(float a, float b) { return __floats2bfloat162_rn(a, b); }
     __device__ static type low2(type v) { return __low2bfloat162(v); }
     __device__ static type high2(type v) { return __high2bfloat162(v); }
@@ -262,6 +271,8 @@ template <> struct Pair<__nv_bfloat16> {
 };
 template <> struct Pair<__half> {
     using type = __half2;
+    __device__ static type abs2(type v) { return __habs2(v); }
+    __device__ static type max2(type a, type b) { return __hmax2(a, b); }
     __device__ static type make(float a, float b) { return __floats2half2_rn(a, b); }
     __device__ static type low2(type v) { return __low2half2(v); }
     __device__ static type high2(type v) { return __high2half2(v); }
@@ -327,47 +338,22 @@ __global__ void __launch_bounds__(kFastThreads) fwht128_stagewise_kernel(const T
                     v[c | st][q] = __hsub2(a, b);
                 }
     // division by sqrt(128) in fp32, one more rounding to the input type
-    const float inv = __frcp_rn(root);
-    const float2 inv2 = make_float2(inv, inv), nroot2 = make_float2(-root, -root);
-    float2 f[8][4];
-    float hi = 0.0f, lo = 3.0e38f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            f[i][j] = P::to_float2(v[i][j]);
-            const float ax = fabsf(f[i][j].x), ay = fabsf(f[i][j].y);
-            hi = fmaxf(hi, fmaxf(ax, ay));
-            lo = fminf(lo, fminf(ax, ay));
-        }
-    if (lo >= 7.888609e-31f && hi <= 1.2676506e30f) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 t = __fmul2_rn(f[i][j], inv2);
-                const float2 rem = __ffma2_rn(t, nroot2, f[i][j]);
-                f[i][j] = __ffma2_rn(rem, inv2, t);
-            }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                f[i][j] = make_float2(div_root(f[i][j].x, root, inv, false), div_root(f[i][j].y, root, inv, false));
-    }
-    float top = 0.0f;
+    const float c128 = quotient_factor(root);
+    const float2 factor = make_float2(c128, c128);
+    T2 most = P::make(0.0f, 0.0f);
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
         T2 o[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            o[q] = P::make(f[c][q].x, f[c][q].y);
-            const float2 r = P::to_float2(o[q]);
-            top = fmaxf(top, fmaxf(fabsf(r.x), fabsf(r.y)));
+            const float2 f = __fmul2_rn(P::to_float2(v[c][q]), factor);
+            o[q] = P::make(f.x, f.y);
+            most = P::max2(most, P::abs2(o[q]));
         }
         if (live) *reinterpret_cast<uint4*>(dst + 8 * (2 * c + h)) = *reinterpret_cast<const uint4*>(o);
     }
+    const float2 most2 = P::to_float2(most);
+    float top = fmaxf(most2.x, most2.y);
     if (amax) {
         if (!live) top = 0.0f;
 #pragma unroll
@@ -384,7 +370,7 @@ __global__ void __launch_bounds__(kFastThreads) fwht128_stagewise_kernel(const T
 }
 
 // Sweep of div_root's reciprocal form against IEEE division: all 2^23 significands of the
-// dividend for both irrational roots.
+// dividend for both irrational roots; and of quotient_factor: every bfloat16 and float16 pattern.
 __global__ void fwht_selftest_kernel(unsigned long long* mismatches) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const float a = __uint_as_float(0x3f800000u | i);
@@ -395,6 +381,15 @@ __global__ void fwht_selftest_kernel(unsigned long long* mismatches) {
         const float inv = __frcp_rn(roots[d]);
         bad += __float_as_uint(div_root(a, roots[d], inv, false)) != __float_as_uint(__fdiv_rn(a, roots[d]));
         bad += __float_as_uint(div_root(-a * 3.0e-5f, roots[d], inv, false)) != __float_as_uint(__fdiv_rn(-a * 3.0e-5f, roots[d]));
+    }
+    if (i < 65536u) {
+        const float factor = quotient_factor(roots[1]);
+        const unsigned short bits = (unsigned short)i;
+        const float vb = __bfloat162float(__ushort_as_bfloat16(bits)), vh = __half2float(__ushort_as_half(bits));
+        const unsigned short qb = __bfloat16_as_ushort(__float2bfloat16_rn(__fdiv_rn(vb, roots[1])));
+        const unsigned short qh = __half_as_ushort(__float2half_rn(__fdiv_rn(vh, roots[1])));
+        bad += vb == vb && qb != __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(vb, factor)));
+        bad += vh == vh && qh != __half_as_ushort(__float2half_rn(__fmul_rn(vh, factor)));
     }
     if (bad) atomicAdd(mismatches, bad);
 }

@@ -283,17 +283,31 @@ __device__ __forceinline__ float error_sum(const float2 (&sq)[8]) {
     return acc;
 }
 // Both candidates of one block.  e2: E2M1, e0: E0M3.
-template <bool kPack, bool kKeep>
+// Two dequantized values: as they are (fp32), or already rounded to a 16-bit type (half the registers).
+template <typename T, int kSize = sizeof(T)> struct Kept;
+template <typename T> struct Kept<T, 4> {
+    using type = float2;
+    __device__ static float2 make(float2 v) { return v; }
+};
+template <typename T> struct Kept<T, 2> {
+    using type = uint32_t;
+    __device__ static uint32_t make(float2 v) {
+        T p[2] = {Elem<T>::round(v.x), Elem<T>::round(v.y)};
+        return *reinterpret_cast<const uint32_t*>(p);
+    }
+};
+template <typename T, bool kPack, bool kKeep>
 struct BlockCandidates {
     uint32_t lo2, hi2, lo0, hi0;     // kPack: level codes of elements 0..7 / 8..15 (E2M1 words with their sign bits)
     uint32_t byte2, byte0;           // E4M3 scale bytes
     float sc2, sc0, err2, err0;
-    float2 d2[8], d0[8];             // kKeep: dequantized values; d2 has the sign of x, a zero of d0 may lack it
+    typename Kept<T>::type d2[8], d0[8];      // kKeep: dequantized values; d2 has the sign of x, a zero of d0 may lack it
 };
 
-// x2[j] = elements (2j, 2j+1) of the block; the packed path.  kWide: x has a full fp32 significand.
-template <bool kWide, bool kPack, bool kKeep>
-__device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs, float rgs, BlockCandidates<kPack, kKeep>& o) {
+// x2[j] = elements (2j, 2j+1) of the block; the packed path.
+template <typename T, bool kPack, bool kKeep>
+__device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs, float rgs, BlockCandidates<T, kPack, kKeep>& o) {
+    constexpr bool kWide = sizeof(T) == 4;
     const float2 rgs2 = make_float2(rgs, rgs), ngs2 = make_float2(-gs, -gs), gs2 = make_float2(gs, gs);
     const float2 neg1 = make_float2(-1.0f, -1.0f);
     float2 s[8];
@@ -314,7 +328,7 @@ __device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs,
             const float2 n = div_rcp2(s[j], nsc2, rsc2);
             byte[j] = __nv_cvt_float2_to_fp4x2(e2m1_nudge_pair(n), __NV_E2M1, cudaRoundNearest);
             const float2 d = __fmul2_rn(__fmul2_rn(e2m1_pair_levels(byte[j]), scv), gs2);
-            if constexpr (kKeep) o.d2[j] = d;
+            if constexpr (kKeep) o.d2[j] = Kept<T>::make(d);
             const float2 e = __ffma2_rn(x2[j], neg1, d);
             sq[j] = __fmul2_rn(e, e);
         }
@@ -347,7 +361,7 @@ __device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs,
                 p4[j >> 1] = (j & 1) == 0 ? __fmaf_rn(fabsf(q.y), 16.0f, fabsf(q.x))
                                           : __fmaf_rn(fabsf(q.y), 4096.0f, __fmaf_rn(fabsf(q.x), 256.0f, p4[j >> 1]));
             const float2 d = __fmul2_rn(__fmul2_rn(q, scv), gs2);
-            if constexpr (kKeep) o.d0[j] = d;
+            if constexpr (kKeep) o.d0[j] = Kept<T>::make(d);
             const float2 e = __ffma2_rn(x2[j], neg1, d);
             sq[j] = __fmul2_rn(e, e);
         }
@@ -360,8 +374,8 @@ __device__ __forceinline__ void candidates_fast(const float2 (&x2)[8], float gs,
 }
 
 // The same with IEEE divisions: any tensor scale, infinities and NaN.
-template <bool kPack, bool kKeep>
-__device__ __noinline__ void candidates_ieee(const float2 (&x2)[8], float gs, BlockCandidates<kPack, kKeep>& o) {
+template <typename T, bool kPack, bool kKeep>
+__device__ __noinline__ void candidates_ieee(const float2 (&x2)[8], float gs, BlockCandidates<T, kPack, kKeep>& o) {
     float s[kGroup], ax[kGroup];
     float amax_s = 0.0f;
     uint32_t sl = 0, sh = 0;                             // sign nibbles of elements 0..7 and 8..15
@@ -381,24 +395,20 @@ __device__ __noinline__ void candidates_ieee(const float2 (&x2)[8], float gs, Bl
     if constexpr (kKeep) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            o.d2[j] = make_float2(x2[j].x < 0.0f ? -d2[2 * j] : d2[2 * j], x2[j].y < 0.0f ? -d2[2 * j + 1] : d2[2 * j + 1]);
-            o.d0[j] = make_float2(d0[2 * j], d0[2 * j + 1]);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float& v = h ? o.d0[j].y : o.d0[j].x;
-                if ((h ? x2[j].y : x2[j].x) < 0.0f) v = -v;
-            }
+            const bool nx = x2[j].x < 0.0f, ny = x2[j].y < 0.0f;
+            o.d2[j] = Kept<T>::make(make_float2(nx ? -d2[2 * j] : d2[2 * j], ny ? -d2[2 * j + 1] : d2[2 * j + 1]));
+            o.d0[j] = Kept<T>::make(make_float2(nx ? -d0[2 * j] : d0[2 * j], ny ? -d0[2 * j + 1] : d0[2 * j + 1]));
         }
     }
 }
 
 template <typename T, bool kPack, bool kKeep>
-__device__ __forceinline__ void block_candidates(const float2 (&x2)[8], float gs, float rgs, bool fast, BlockCandidates<kPack, kKeep>& o) {
-    if (fast) candidates_fast<sizeof(T) == 4>(x2, gs, rgs, o);
+__device__ __forceinline__ void block_candidates(const float2 (&x2)[8], float gs, float rgs, bool fast, BlockCandidates<T, kPack, kKeep>& o) {
+    if (fast) candidates_fast(x2, gs, rgs, o);
     // a NaN (or a value whose quotient overflows) leaves the packed path with a NaN or an infinity in the error
     if (!fast || !(__fadd_rn(o.err2, o.err0) < __int_as_float(0x7f800000))) {
         float2 copy[8];                                  // copies: only these have addresses, o stays in registers
-        BlockCandidates<kPack, kKeep> t;
+        BlockCandidates<T, kPack, kKeep> t;
 #pragma unroll
         for (int j = 0; j < 8; ++j) copy[j] = x2[j];
         candidates_ieee(copy, gs, t);
@@ -454,16 +464,13 @@ __device__ __forceinline__ void load_block(const T* src, int left, bool vec, boo
 // The chosen candidate's dequantized values, rounded to T.  16-bit types: both candidates as packed pairs, the
 // E0M3 pair takes its signs from the E2M1 pair (a negative element that rounds to zero gives -0 in either format).
 template <typename T, bool kPack>
-__device__ __forceinline__ void store_block(T* out, int left, bool vec, bool use_e0, const BlockCandidates<kPack, true>& o) {
+__device__ __forceinline__ void store_block(T* out, int left, bool vec, bool use_e0, const BlockCandidates<T, kPack, true>& o) {
     T vals[kGroup];
     if constexpr (sizeof(T) == 2) {
         uint32_t* v = reinterpret_cast<uint32_t*>(vals);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            T p2[2] = {Elem<T>::round(o.d2[j].x), Elem<T>::round(o.d2[j].y)};
-            T p0[2] = {Elem<T>::round(o.d0[j].x), Elem<T>::round(o.d0[j].y)};
-            const uint32_t w2 = *reinterpret_cast<const uint32_t*>(p2), w0 = *reinterpret_cast<const uint32_t*>(p0);
-            v[j] = use_e0 ? (w0 | (w2 & 0x80008000u)) : w2;
+            v[j] = use_e0 ? (o.d0[j] | (o.d2[j] & 0x80008000u)) : o.d2[j];
         }
     } else {
 #pragma unroll
@@ -611,7 +618,7 @@ __global__ void selftest_e2m1_kernel(unsigned long long* mismatches) {
 // walks over (row, 64-block chunk) items with the grid's stride; a lane takes the blocks lane and
 // lane + 32 of an item, so the index arithmetic of an item is shared by two blocks.
 template <typename T, bool kPack, bool kDequant>
-__global__ void __launch_bounds__(kThreads, (kPack && !kDequant) ? 3 : 2) quantize_kernel(const QuantArgs a) {
+__global__ void __launch_bounds__(kThreads, !kDequant || (!kPack && sizeof(T) == 2) ? 3 : 2) quantize_kernel(const QuantArgs a) {
     // a kernel launched behind this one with programmatic dependent launch (the W4A4 GEMM) may set itself up
     // while this grid runs; it waits for this grid's end before it reads the outputs
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -647,7 +654,7 @@ __global__ void __launch_bounds__(kThreads, (kPack && !kDequant) ? 3 : 2) quanti
             const int left = (int)min((int64_t)kGroup, a.k - c0);
             float2 x2[8];
             load_block(static_cast<const T*>(a.x) + row * a.ldx + c0, left, a.vec_in, a.in_place, x2);
-            BlockCandidates<kPack, kDequant> o;
+            BlockCandidates<T, kPack, kDequant> o;
             block_candidates<T>(x2, gs, rgs, fast, o);
             if (a.mode != MIXFP4_MODE_GIVEN)
                 use_e0 = a.mode == MIXFP4_MODE_ORACLE16 ? (o.err0 < o.err2) : (a.mode == MIXFP4_MODE_ALL_E0M3);
@@ -688,7 +695,7 @@ __global__ void __launch_bounds__(kThreads, (kPack && !kDequant) ? 3 : 2) quanti
 // Rows past the tensor and blocks past K get what an all-zero block quantizes to.  CTA 0 also writes the weight's
 // decode table.  Bound by instruction issue like the kernel above.  Loading a rotated 14336 x 4096 bf16 projection
 // (rotation with the maximum in the same pass, this kernel, nothing else): 169 us, against 220 us for rotation, amax,
-// canonical quantizer, repack and table launch.
+// canonical quantizer, repack and table launch (127 us since the rotation divides by one multiplication).
 struct StreamQuantArgs {
     const void* x;
     int64_t rows, k, ldx, groups, subs, items;       // items = row tiles * subs * 4
@@ -726,7 +733,7 @@ __global__ void __launch_bounds__(kThreads, 3) quantize_stream_kernel(const Stre
             const int64_t c0 = blk * kGroup;
             float2 x2[8];
             load_block(static_cast<const T*>(a.x) + row * a.ldx + c0, (int)min((int64_t)kGroup, a.k - c0), a.vec_in, false, x2);
-            BlockCandidates<true, false> o;
+            BlockCandidates<T, true, false> o;
             block_candidates<T>(x2, gs, rgs, fast, o);
             const bool use_e0 = a.mode == MIXFP4_MODE_ORACLE16 ? (o.err0 < o.err2) : (a.mode == MIXFP4_MODE_ALL_E0M3);
             lo = codes_to_kernel_layout(use_e0 ? o.lo0 | (o.lo2 & 0x88888888u) : o.lo2);
@@ -755,7 +762,7 @@ struct RegionArgs {
     int64_t ldo;
 };
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) fake_regions_kernel(const RegionArgs a) {
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) fake_regions_kernel(const RegionArgs a) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float e2[kThreads], e0[kThreads], s2[kThreads], s0[kThreads];
     __shared__ uint8_t pick[kThreads];
@@ -769,7 +776,7 @@ __global__ void __launch_bounds__(kThreads, 2) fake_regions_kernel(const RegionA
         const int64_t row = tile_r * tr + r, blk = tile_g * tg + g, c0 = blk * kGroup;
         const bool real = row < a.rows && blk < a.groups;
         const int left = real ? (int)min((int64_t)kGroup, a.k - c0) : 0;
-        BlockCandidates<false, true> o;
+        BlockCandidates<T, false, true> o;
         o.err2 = o.err0 = 0.0f;                       // cells past the tensor's edge count as zero
         if (real) {
             float2 x2[8];
