@@ -92,7 +92,7 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
     if out_dtype not in (torch.float32, torch.bfloat16):
         raise TypeError("out_dtype must be float32 or bfloat16")
     lead = x.shape[:-1]
-    x2 = x.reshape(-1, packed.k)
+    x2 = x if x.dim() == 2 else x.reshape(-1, packed.k)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     m = x2.shape[0]
@@ -119,7 +119,7 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
         if fusable:
             nbytes = lib.mixfp4_gemm_workspace_bytes(m, packed.n, packed.k)
             ws = _workspace(x.device, nbytes)
-            with torch.cuda.device(x.device):
+            with nat.on_device(x.device):
                 st = lib.mixfp4_gemm_a4(x2.data_ptr(), m, x2.stride(0), packed.codes.data_ptr(), packed.scales.data_ptr(),
                                         nat.ptr(packed.fmt), packed.global_scale.data_ptr(), packed.n, packed.k,
                                         packed.layout_code, nat.ptr(packed.lut), 128 if spec is not None else 0,
@@ -134,7 +134,7 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
             x2 = _rotation.apply_transform(x2, spec, rounding="reference")
             spec = None
         x2 = fake_quantize_activations(x2, act)
-    with torch.cuda.device(x.device):
+    with nat.on_device(x.device):
         stream = nat.stream_ptr(x.device)
         if m <= GEMV_MAX_M:
             if spec is not None:
@@ -161,7 +161,7 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
             nat.check("mixfp4_gemm", st)
     if bias is not None:
         y += bias.to(y.dtype)
-    return y.reshape(*lead, packed.n)
+    return y if x.dim() == 2 else y.reshape(*lead, packed.n)
 
 
 def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dtype: torch.dtype | None = None,
@@ -193,7 +193,7 @@ def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dty
             seg.codes, seg.scales, seg.global_scale = p.codes.data_ptr(), nat.ptr(p.scales), p.global_scale.data_ptr()
             seg.lut, seg.y, seg.ldy, seg.n = nat.ptr(p.lut), y.data_ptr(), y.stride(0), p.n
         flags = nat.gemv_flags(overlap_previous, *[p.lut for p in packs])
-        with torch.cuda.device(x.device):
+        with nat.on_device(x.device):
             tma_rows = x2.data_ptr() % 16 == 0 and x2.stride(0) % 8 == 0        # a tensor map can address them
             if m <= GEMV_MAX_M:
                 fn = "mixfp4_gemv_grouped"

@@ -29,6 +29,7 @@ TAIL_POLICY = (
     "partial_N_or_M_and_K_format_regions_use_only_real_K16_blocks"
 )
 
+_LAYOUT_CODE = {"canonical": nat.LAYOUT_CANONICAL, "kernel": nat.LAYOUT_KERNEL, "stream": nat.LAYOUT_STREAM}
 _MODE_CODE = {"oracle16": nat.MODE_ORACLE16, "all_e2m1": nat.MODE_ALL_E2M1, "all_e0m3": nat.MODE_ALL_E0M3}
 # coarse format regions (project_quant/region.py:42-70): name -> (rows, K16 blocks) of a region
 # (rows, 0) stands for "layer": one format for the whole tensor
@@ -91,7 +92,7 @@ class PackedWeight:
 
     @property
     def layout_code(self) -> int:
-        return {"canonical": nat.LAYOUT_CANONICAL, "kernel": nat.LAYOUT_KERNEL, "stream": nat.LAYOUT_STREAM}[self.layout]
+        return _LAYOUT_CODE[self.layout]
 
     def format_ids(self) -> torch.Tensor:
         """uint8 [n, ceil(k/16)], 1 = E0M3 (GranularityResult.format_ids of the reference)."""
@@ -134,7 +135,7 @@ class PackedWeight:
         if self.lut is None or (wide and self.lut.numel() < nat.WIDE_TABLE_BYTES):
             lut = torch.empty(nat.WIDE_TABLE_BYTES if wide else 4096, dtype=torch.uint8, device=self.device)
             fn = nat.lib().mixfp4_decode_table_wide if wide else nat.lib().mixfp4_decode_table
-            with torch.cuda.device(self.device):
+            with nat.on_device(self.device):
                 st = fn(self.global_scale.data_ptr(), lut.data_ptr(), nat.stream_ptr(self.device))
             nat.check("mixfp4_decode_table", st)
             self.lut = lut
@@ -147,7 +148,7 @@ class PackedWeight:
             src = self if self.layout == "canonical" else self._repack("canonical")
             lib = nat.lib()
             chunks = torch.empty(lib.mixfp4_stream_bytes(self.n, self.k), dtype=torch.uint8, device=self.device)
-            with torch.cuda.device(self.device):
+            with nat.on_device(self.device):
                 st = lib.mixfp4_repack_stream(src.codes.data_ptr(), src.scales.data_ptr(), src.fmt.data_ptr(), self.n,
                                               self.k, chunks.data_ptr(), nat.stream_ptr(self.device))
             nat.check("mixfp4_repack_stream", st)
@@ -157,7 +158,7 @@ class PackedWeight:
             codes = torch.empty((self.n, self.kpad // 2), dtype=torch.uint8, device=self.device)
             scales = torch.empty((self.n, self.kpad // 16), dtype=torch.uint8, device=self.device)
             fmt = torch.empty((self.n, self.kpad // 128), dtype=torch.uint8, device=self.device)
-            with torch.cuda.device(self.device):
+            with nat.on_device(self.device):
                 st = nat.lib().mixfp4_repack_from_stream(self.codes.data_ptr(), self.n, self.k, codes.data_ptr(),
                                                          scales.data_ptr(), fmt.data_ptr(), nat.stream_ptr(self.device))
             nat.check("mixfp4_repack_from_stream", st)
@@ -165,7 +166,7 @@ class PackedWeight:
             return canon if to == "canonical" else canon._repack(to)
         codes, scales = torch.empty_like(self.codes), torch.empty_like(self.scales)
         fmt = None if to == "kernel" else torch.empty((self.n, self.kpad // 128), dtype=torch.uint8, device=self.device)
-        with torch.cuda.device(self.device):
+        with nat.on_device(self.device):
             st = nat.lib().mixfp4_repack(self.codes.data_ptr(), self.scales.data_ptr(), nat.ptr(self.fmt), self.n, self.k,
                                          nat.LAYOUT_KERNEL if to == "kernel" else nat.LAYOUT_CANONICAL,
                                          codes.data_ptr(), scales.data_ptr(), nat.ptr(fmt), nat.stream_ptr(self.device))
@@ -253,7 +254,7 @@ def validate_layout(x: torch.Tensor, *, scale_group_size: int, operand_role: str
 def tensor_amax(x2: torch.Tensor) -> torch.Tensor:
     """max |x| of a 2-D CUDA tensor as a float32 [1] device tensor (no host sync)."""
     out = torch.empty(1, dtype=torch.float32, device=x2.device)
-    with torch.cuda.device(x2.device):
+    with nat.on_device(x2.device):
         st = nat.lib().mixfp4_amax(x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], x2.shape[0], x2.shape[1],
                                    x2.stride(0), out.data_ptr(), nat.stream_ptr(x2.device))
     nat.check("mixfp4_amax", st)
@@ -310,7 +311,7 @@ def quantize_packed(x: torch.Tensor, *, mode: str = "oracle16", amax: torch.Tens
             raise NotImplementedError("coarse regions over several rows need more than one region along K")
         e2e = stats["e2_errors"] if stats else torch.empty((rows, groups), dtype=torch.float32, device=dev)
         e0e = stats["e0_errors"] if stats else torch.empty((rows, groups), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with nat.on_device(dev):
             st = nat.lib().mixfp4_quantize(
                 x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], rows, k, x2.stride(0), nat.MODE_ORACLE16, amax.data_ptr(),
                 codes.data_ptr(), scales.data_ptr(), fmt.data_ptr(), gs.data_ptr(), e2e.data_ptr(), e0e.data_ptr(),
@@ -325,7 +326,7 @@ def quantize_packed(x: torch.Tensor, *, mode: str = "oracle16", amax: torch.Tens
                 st = nat.lib().mixfp4_select_regions(e2e.data_ptr(), e0e.data_ptr(), rows, k, region[0], region[1],
                                                      fmt.data_ptr(), nat.stream_ptr(dev))
                 nat.check("mixfp4_select_regions", st)
-    with torch.cuda.device(dev):
+    with nat.on_device(dev):
         st = nat.lib().mixfp4_quantize(
             x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], rows, k, x2.stride(0), mode_code, amax.data_ptr(),
             codes.data_ptr(), scales.data_ptr(), fmt.data_ptr(), gs.data_ptr(),
@@ -351,7 +352,7 @@ def quantize_stream(x: torch.Tensor, *, mode: str = "oracle16", amax: torch.Tens
     chunks = torch.empty(lib.mixfp4_stream_bytes(rows, k), dtype=torch.uint8, device=dev)
     lut = torch.empty(nat.WIDE_TABLE_BYTES, dtype=torch.uint8, device=dev)
     gs = torch.empty(1, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with nat.on_device(dev):
         st = lib.mixfp4_quantize_stream(x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], rows, k, x2.stride(0), _MODE_CODE[mode],
                                         amax.data_ptr(), chunks.data_ptr(), gs.data_ptr(), lut.data_ptr(),
                                         nat.stream_ptr(dev))
@@ -367,7 +368,7 @@ def _codebook(x: torch.Tensor, e0m3: bool) -> torch.Tensor:
     xf = (xf.cuda() if host_input else xf).contiguous()
     out = torch.empty_like(xf)
     if xf.numel():
-        with torch.cuda.device(xf.device):
+        with nat.on_device(xf.device):
             st = nat.lib().mixfp4_round_codebook(xf.data_ptr(), out.data_ptr(), xf.numel(), int(e0m3),
                                                  nat.stream_ptr(xf.device))
         nat.check("mixfp4_round_codebook", st)
@@ -520,7 +521,7 @@ def build_scaled_candidate(grouped: torch.Tensor, *, format_name: str, global_sc
     exp = torch.empty(lead, dtype=torch.uint8, device=g.device)
     if nblocks:
         amax = tensor_amax(g.reshape(-1, SCALE_GROUP_SIZE))
-        with torch.cuda.device(g.device):
+        with nat.on_device(g.device):
             st = nat.lib().mixfp4_e0_four_over_six(g.data_ptr(), nblocks, amax.data_ptr(), codes.data_ptr(), deq.data_ptr(),
                                                    scales.data_ptr(), errors.data_ptr(), exp.data_ptr(),
                                                    nat.stream_ptr(g.device))
@@ -563,7 +564,7 @@ def _fake_quantize(x: torch.Tensor, mode: str, region: tuple[int, int] | None, i
     amax = torch.empty(1, dtype=torch.float32, device=x2.device)
     head = (x2.data_ptr(), nat.DTYPE_CODE[x2.dtype], rows, k, x2.stride(0))
     tail = (amax.data_ptr(), out.data_ptr(), out.stride(0), nat.stream_ptr(x2.device))
-    with torch.cuda.device(x2.device):
+    with nat.on_device(x2.device):
         if region is None:
             nat.check("mixfp4_fake_quantize", nat.lib().mixfp4_fake_quantize(*head, _MODE_CODE[mode], *tail))
         else:
@@ -580,7 +581,7 @@ def dequantize(packed: PackedWeight, dtype: torch.dtype = torch.bfloat16) -> tor
         raise TypeError("dtype must be bfloat16, float16 or float32")
     nat.require_cuda(packed.codes, "packed weight")
     out = torch.empty((packed.n, packed.k), dtype=dtype, device=packed.device)
-    with torch.cuda.device(packed.device):
+    with nat.on_device(packed.device):
         st = nat.lib().mixfp4_dequant(packed.codes.data_ptr(), packed.scales.data_ptr(), nat.ptr(packed.fmt),
                                       packed.global_scale.data_ptr(), packed.n, packed.k, packed.layout_code,
                                       out.data_ptr(), nat.DTYPE_CODE[dtype], packed.k, nat.stream_ptr(packed.device))

@@ -81,7 +81,7 @@ def _run_fwht(x: torch.Tensor, size: int, signs: torch.Tensor | None, stagewise:
     dst = out if out is not None else torch.empty_like(src)
     args = (src.data_ptr(), dst.data_ptr(), nat.DTYPE_CODE[src.dtype], rows, k, k, k, size, nat.ptr(signs),
             1 if stagewise else 0)
-    with torch.cuda.device(src.device):
+    with nat.on_device(src.device):
         if amax is None:
             st = nat.lib().mixfp4_fwht(*args, nat.stream_ptr(src.device))
         else:                                       # float32 [1] on the device: the largest magnitude of the result
