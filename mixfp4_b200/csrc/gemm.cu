@@ -494,8 +494,6 @@ struct PairCfg {
     // kind::f16 instruction descriptor as above with M = 256 (the pair), N = 256
     static constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                                            ((uint32_t)(256 >> 4) << 24);
-    static constexpr int kThreadsPerRow = kDecodeWarps * 32 / BNH;   // 2
-    static constexpr int kWords = 8 / kThreadsPerRow;                // 4
 };
 
 // Arrive on the leader CTA's copy of a barrier (from either CTA of the pair).
@@ -593,13 +591,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_a(s), 1);                    // leader: its own expect_tx arrival; bytes of both CTAs
-            mbar_init(full_b(s), 2 * kDecodeWarps);     // leader: the transcoder warps of both CTAs
+            mbar_init(full_b(s), kDecodeWarps);         // leader: the stage's transcoder group in both CTAs
             mbar_init(empty(s), 1);                     // each CTA: the leader's commit
         }
         mbar_init(accum_bar, 1);
         for (int s = 0; s < kWStages; ++s) {
             mbar_init(full_w(s), 1);
-            mbar_init(empty_w(s), kDecodeWarps);
+            mbar_init(empty_w(s), kDecodeWarps / 2);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -683,9 +681,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
         }
     } else {
         // -------------------------------------------------- weight transcoders / epilogue
-        constexpr int kWords = C::kWords, kBlocks = kWords / 2, kTPR = C::kThreadsPerRow;
-        const int dt = threadIdx.x - 64;                // transcoder thread index
-        const int row = dt / kTPR, part = dt % kTPR;    // row of this CTA's half tile, part of the K step
+        // Two groups of four warps take the K steps in turn, a thread a whole row of the half tile: the waits, table
+        // look-ups and fences of one step run under the other group's decode (all eight warps on every step: 4096 x 14336
+        // at 777 tokens 121 us, so 89; 28672 x 8192 at 4096 tokens 1490 and 1471).
+        static_assert(kStages % 2 == 0 && kWStages % 2 == 0, "a stage belongs to one transcoder group");
+        const int grp = (warp - 2) >> 2, row = ((warp - 2) & 3) * 32 + lane;
         const uint32_t last_row = (uint32_t)a.n - 1;
         const uint32_t grow = min(nh0 + row, last_row);
         const uint8_t* srow = a.stream_layout
@@ -696,62 +696,51 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
         const uint32_t lut_base = base + C::kOffLut;
         const uint32_t row_off = (row >> 3) * 1024u + (row & 7) * 128u;
         const uint32_t sw = row & 7;
-
-        auto load_codes = [&](uint32_t (&w)[kWords], int kt) -> bool {
-            const int ws = kt % kWStages;
-            if (!__all_sync(0xffffffffu, mbar_wait(full_w(ws), (kt / kWStages) & 1, ctx, 9))) return false;
-            const uint32_t src = base + C::kOffW + ws * C::kWBytes + row * 32 + part * (kWords * 4);
-            if constexpr (kWords == 4) {
-                const uint4 v = lds128_lut(src);
-                w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-            } else {
-                asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(src));
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty_w(ws));
-            return true;
+        const int pairs = num_kt >> 1;                  // num_kt is even; a row's scale word of a step: four blocks
+        auto load_scales = [&](int pair) -> uint32_t {
+            return __ldg(reinterpret_cast<const uint32_t*>(srow + (size_t)pair * sstep + 4 * grp));
         };
-        auto load_scale_pair = [&](int pair) -> uint2 { return __ldg(reinterpret_cast<const uint2*>(srow + (size_t)pair * sstep)); };
 
-        uint32_t codes[kWords], ncodes[kWords];
-        bool ok = load_codes(codes, 0);
-        uint2 sc2 = load_scale_pair(0), nsc2 = num_kt > 2 ? load_scale_pair(1) : sc2, nnsc2 = nsc2;   // two pairs ahead
+        bool ok = true;
+        uint32_t sc = load_scales(0), nsc = pairs > 1 ? load_scales(1) : sc;     // fetched two steps of the group ahead
         uint32_t fb = kKL ? 0u : __ldg(fptr);
-        for (int kt = 0; kt < num_kt && ok; ++kt) {
-            const int s = kt % kStages;
+        for (int kt = grp; kt < num_kt; kt += 2) {
+            const int s = kt % kStages, ws = kt % kWStages, pair = kt >> 1;
             const uint32_t ph = (kt / kStages) & 1;
-            uint32_t nfb = fb;
-            if (kt + 1 < num_kt) {
-                ok = load_codes(ncodes, kt + 1);
-                if (!ok) break;
-                if ((kt & 1) == 0 && kt + 4 < num_kt) nnsc2 = load_scale_pair((kt >> 1) + 2);
-                if constexpr (!kKL) nfb = __ldg(fptr + ((kt + 1) >> 1));
-            }
-            const uint32_t scs = ((kt & 1) ? sc2.y : sc2.x) >> (8 * part * kBlocks);
+            const uint32_t nnsc = pair + 2 < pairs ? load_scales(pair + 2) : nsc;
+            const uint32_t nfb = !kKL && pair + 1 < pairs ? __ldg(fptr + pair + 1) : fb;
+            ok = __all_sync(0xffffffffu, mbar_wait(full_w(ws), (kt / kWStages) & 1, ctx, 9));
+            if (!ok) break;
+            // the row's 32 bytes of codes, the halves in an order that spreads the banks
+            const uint32_t src = base + C::kOffW + ws * C::kWBytes + row * 32;
+            const uint32_t c0 = (lane >> 2) & 1;
+            const uint4 va = lds128_lut(src + c0 * 16), vb = lds128_lut(src + (c0 ^ 1) * 16);
+            const uint4 lo = c0 ? vb : va, hi = c0 ? va : vb;
+            const uint32_t codes[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
             ok = __all_sync(0xffffffffu, mbar_wait_cluster(empty(s), ph ^ 1, ctx, 5));
             if (!ok) break;
             const uint32_t dst = base + C::kOffB + s * C::kBBytes + row_off;
-            const uint32_t fbits = fb >> ((kt & 1) * 4 + part * kBlocks);
 #pragma unroll
-            for (int b = 0; b < kBlocks; ++b) {
-                const uint32_t idx = kKL ? ((scs >> (8 * b)) & 0xffu)
-                                         : ((((fbits >> b) & 1u) << 7) | ((scs >> (8 * b)) & 0x7fu));
+            for (int b = 0; b < 4; ++b) {
+                const uint32_t idx = kKL ? ((sc >> (8 * b)) & 0xffu)
+                                         : ((((fb >> (4 * grp + b)) & 1u) << 7) | ((sc >> (8 * b)) & 0x7fu));
                 const uint4 tab = lds128_lut(lut_base + idx * 16);
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
                     const int i = 2 * b + w;
                     uint32_t p[4];
                     decode_word<kKL>(codes[i], tab, p);
-                    const uint32_t chunk = (uint32_t)(part * kWords + i) ^ sw;
-                    sts128(dst + chunk * 16, p[0], p[1], p[2], p[3]);
+                    sts128(dst + (((uint32_t)i ^ sw) * 16), p[0], p[1], p[2], p[3]);
                 }
             }
             fence_async_proxy();
             __syncwarp();
-            if (lane == 0) mbar_arrive_leader(full_b(s));   // this CTA's half is in place
-#pragma unroll
-            for (int i = 0; i < kWords; ++i) codes[i] = ncodes[i];
-            if (kt & 1) { sc2 = nsc2; nsc2 = nnsc2; }
+            if (lane == 0) {
+                mbar_arrive(empty_w(ws));               // every word has been used
+                mbar_arrive_leader(full_b(s));          // this CTA's half is in place
+            }
+            sc = nsc;
+            nsc = nnsc;
             fb = nfb;
         }
 
