@@ -12,9 +12,9 @@
 //               tcgen05.mma.cta_group::1.kind::f16 (128x128x16, bf16 x bf16 -> fp32) per
 //               stage and commits the stage's "empty" barrier; after the last K step it
 //               commits the accumulator barrier.
-//   warps 2-9   weight transcoders, then epilogue.  Each thread owns half a row of the
-//               128 x 64 weight tile (a whole row of a 256-row tile): it reads 16 or 32 B of
-//               codes from the shared-memory code ring one K step ahead, takes its scale bytes (8 B per row and two K steps)
+//   warps 2-9   weight transcoders, then epilogue.  Each thread owns a row of the weight tile's
+//               K step (128-row tiles: two groups of four warps take the steps in turn): it reads 32 B of
+//               codes from the shared-memory code ring, takes its scale bytes (8 B per row and two K steps)
 //               straight from global memory, decodes with the shared (format, scale) ->
 //               bf16 table into exactly the reference's dequantized bf16 values and writes
 //               them into the K-major 128B-swizzled operand layout tcgen05 reads
@@ -76,9 +76,9 @@ struct Cfg {
     // and 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
     static constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) |
                                            ((uint32_t)(128 >> 4) << 24);
-    // transcoders: 256 threads over kBN rows
-    static constexpr int kThreadsPerRow = kDecodeWarps * 32 / kBN;   // 2 or 1
-    static constexpr int kWords = 8 / kThreadsPerRow;           // 32-bit code words per thread and K step: 4 or 8
+    // transcoders: a row of the tile per thread; with 128 rows two groups of warps take the K steps in turn
+    static constexpr int kGroups = kDecodeWarps * 32 / kBN;     // 2 or 1
+    static constexpr int kStepWarps = kDecodeWarps / kGroups;
 };
 
 struct GemmArgs {
@@ -199,13 +199,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_a(s), 1);
-            mbar_init(full_b(s), kDecodeWarps);
+            mbar_init(full_b(s), C::kStepWarps);
             mbar_init(empty(s), 1);
         }
         mbar_init(accum_bar, 1);
         for (int s = 0; s < kWStages; ++s) {
             mbar_init(full_w(s), 1);
-            mbar_init(empty_w(s), kDecodeWarps);
+            mbar_init(empty_w(s), C::kStepWarps);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -285,12 +285,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         }
     } else {
         // -------------------------------------------------- weight transcoders / epilogue
-        constexpr int kWords = C::kWords, kBlocks = kWords / 2;
-        // The threads of a row are neighbouring lanes, so a warp reads whole 32-byte code rows
-        // (conflict-free) and its 16-byte stores into the swizzled tile never share a bank.
-        constexpr int kTPR = C::kThreadsPerRow;
-        const int dt = threadIdx.x - 64;                // transcoder thread index
-        const int row = dt / kTPR, part = dt % kTPR;    // tile row, which part of the K step
+        // A thread decodes a whole row of a K step.  256-row tiles: all eight warps work on every step.  128-row tiles:
+        // two groups of four warps take the steps in turn, so that the waits, look-ups and fences of one step run under
+        // the other group's decode (14336 x 4096 at 256 tokens 44.0 -> 39.0 us, 4096 x 4096 at 512 32.9 -> 28.8 us).
+        constexpr int kGroups = C::kGroups;
+        static_assert(kStages % kGroups == 0 && (kWStages % kGroups == 0), "a stage belongs to one transcoder group");
+        const int grp = kGroups == 2 ? (warp - 2) >> 2 : 0;
+        const int row = (kGroups == 2 ? ((warp - 2) & 3) : warp - 2) * 32 + lane;
         const uint32_t last_row = (uint32_t)a.n - 1;
         const uint32_t grow = min(n0 + row, last_row);  // rows past N re-read the last row; never stored
         // a row's 8 scale bytes per 128 K elements: 8 bytes apart in a scale row, one chunk apart in the stream layout
@@ -303,75 +304,53 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         // destination of this thread's 16-byte chunks: row r, logical chunk c -> c ^ (r & 7)
         const uint32_t row_off = (row >> 3) * 1024u + (row & 7) * 128u;
         const uint32_t sw = row & 7;
+        const int pair0 = kt0 >> 1, pairs = (num_kt + 1) >> 1;         // 128 K elements: two steps (kt0 is even)
+        auto load_scales = [&](int pair) -> uint2 { return __ldg(reinterpret_cast<const uint2*>(srow + (size_t)(pair0 + pair) * sstep)); };
 
-        // The code tile of a K step is in shared memory (32 bytes per row, rows past N zero-filled
-        // by TMA).
-        auto load_codes = [&](uint32_t (&w)[kWords], int kt) -> bool {
-            const int ws = kt % kWStages;
-            if (!__all_sync(0xffffffffu, mbar_wait(full_w(ws), (kt / kWStages) & 1, ctx, 9))) return false;
-            const uint32_t src = base + C::kOffW + ws * C::kWBytes + row * 32 + part * (kWords * 4);
-            if constexpr (kWords == 8) {   // one thread per row: read the halves in an order that spreads the banks
-                const uint32_t c0 = (lane >> 2) & 1;
-                const uint4 va = lds128_lut(src + c0 * 16), vb = lds128_lut(src + (c0 ^ 1) * 16);
-                const uint4 lo = c0 ? vb : va, hi = c0 ? va : vb;
-                w[0] = lo.x; w[1] = lo.y; w[2] = lo.z; w[3] = lo.w;
-                w[4] = hi.x; w[5] = hi.y; w[6] = hi.z; w[7] = hi.w;
-            } else if constexpr (kWords == 4) {
-                const uint4 v = lds128_lut(src);
-                w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-            } else {
-                asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(src));
-            }
-            __syncwarp();                               // every lane has read: the stage may be refilled
-            if (lane == 0) mbar_arrive(empty_w(ws));
-            return true;
-        };
-        // Scales: 8 bytes of a row cover two K steps.
-        auto load_scale_pair = [&](int pair) -> uint2 {
-            return __ldg(reinterpret_cast<const uint2*>(srow + (size_t)pair * sstep));
-        };
-
-        uint32_t codes[kWords], ncodes[kWords];
-        bool ok = load_codes(codes, 0);
-        // scale pairs are fetched two pairs (four K steps) ahead: a global load takes longer than two steps
-        uint2 sc2 = load_scale_pair(kt0 >> 1), nsc2 = num_kt > 2 ? load_scale_pair((kt0 >> 1) + 1) : sc2, nnsc2 = nsc2;
-        uint32_t fb = kKL ? 0u : __ldg(fptr + (kt0 >> 1));
-        for (int kt = 0; kt < num_kt && ok; ++kt) {
-            const int s = kt % kStages;
+        bool ok = true;
+        // scale pairs are fetched two pairs ahead: a global load takes longer than a step
+        uint2 sc2 = load_scales(0), nsc2 = pairs > 1 ? load_scales(1) : sc2, nnsc2 = nsc2;
+        uint32_t fb = kKL ? 0u : __ldg(fptr + pair0), nfb = fb;
+        for (int kt = grp; kt < num_kt; kt += kGroups) {
+            const int s = kt % kStages, ws = kt % kWStages, pair = kt >> 1;
             const uint32_t ph = (kt / kStages) & 1;
-            uint32_t nfb = fb;
-            if (kt + 1 < num_kt) {                      // next K step's packed data, one step ahead
-                ok = load_codes(ncodes, kt + 1);
-                if (!ok) break;
-                if ((kt & 1) == 0 && kt + 4 < num_kt) nnsc2 = load_scale_pair(((kt0 + kt) >> 1) + 2);
-                if constexpr (!kKL) nfb = __ldg(fptr + ((kt0 + kt + 1) >> 1));
+            if (kGroups == 2 || (kt & 1) == 0) {
+                nnsc2 = pair + 2 < pairs ? load_scales(pair + 2) : nsc2;
+                if constexpr (!kKL) nfb = pair + 1 < pairs ? __ldg(fptr + pair0 + pair + 1) : fb;
             }
-            const uint32_t scs = ((kt & 1) ? sc2.y : sc2.x) >> (8 * part * kBlocks);
+            // The code tile of a K step is in shared memory (32 bytes per row, rows past N zero-filled by TMA): the halves
+            // are read in an order that spreads the banks.
+            ok = __all_sync(0xffffffffu, mbar_wait(full_w(ws), (kt / kWStages) & 1, ctx, 9));
+            if (!ok) break;
+            const uint32_t src = base + C::kOffW + ws * C::kWBytes + row * 32;
+            const uint32_t c0 = (lane >> 2) & 1;
+            const uint4 va = lds128_lut(src + c0 * 16), vb = lds128_lut(src + (c0 ^ 1) * 16);
+            const uint4 lo = c0 ? vb : va, hi = c0 ? va : vb;
+            const uint32_t codes[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
             ok = __all_sync(0xffffffffu, mbar_wait(empty(s), ph ^ 1, ctx, 5));   // warp-uniform: lanes stay together
             if (!ok) break;
+            const uint32_t sc = (kt & 1) ? sc2.y : sc2.x;
             const uint32_t dst = base + C::kOffB + s * C::kBBytes + row_off;
-            const uint32_t fbits = fb >> ((kt & 1) * 4 + part * kBlocks);     // this thread's blocks
 #pragma unroll
-            for (int b = 0; b < kBlocks; ++b) {
-                const uint32_t idx = kKL ? ((scs >> (8 * b)) & 0xffu)
-                                         : ((((fbits >> b) & 1u) << 7) | ((scs >> (8 * b)) & 0x7fu));
+            for (int b = 0; b < 4; ++b) {
+                const uint32_t idx = kKL ? ((sc >> (8 * b)) & 0xffu)
+                                         : ((((fb >> ((kt & 1) * 4 + b)) & 1u) << 7) | ((sc >> (8 * b)) & 0x7fu));
                 const uint4 tab = lds128_lut(lut_base + idx * 16);
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
                     const int i = 2 * b + w;
                     uint32_t p[4];
                     decode_word<kKL>(codes[i], tab, p);
-                    const uint32_t chunk = (uint32_t)(part * kWords + i) ^ sw;
-                    sts128(dst + chunk * 16, p[0], p[1], p[2], p[3]);
+                    sts128(dst + (((uint32_t)i ^ sw) * 16), p[0], p[1], p[2], p[3]);
                 }
             }
             fence_async_proxy();                        // generic-proxy stores -> visible to tcgen05
             __syncwarp();
-            if (lane == 0) mbar_arrive(full_b(s));
-#pragma unroll
-            for (int i = 0; i < kWords; ++i) codes[i] = ncodes[i];
-            if (kt & 1) { sc2 = nsc2; nsc2 = nnsc2; }
-            fb = nfb;
+            if (lane == 0) {
+                mbar_arrive(empty_w(ws));               // every word has been used
+                mbar_arrive(full_b(s));
+            }
+            if (kGroups == 2 || (kt & 1)) { sc2 = nsc2; nsc2 = nnsc2; fb = nfb; }
         }
 
         if (ok && mbar_wait(accum_bar, 0, ctx, 6)) {
