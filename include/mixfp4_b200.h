@@ -152,7 +152,8 @@ MIXFP4_API int mixfp4_select_layer(const float* e2_err, const float* e0_err, int
 /* Diagnostic: the quantizer divides by block scales with a reciprocal-and-residual sequence
  * instead of a full IEEE division.  This runs the exhaustive proof that the two agree (all 2^23
  * dividend significands x the 8 significands an E4M3 scale or the constants 6 and 7 can have;
- * likewise for the Hadamard kernel's division by sqrt(32) and sqrt(128)), and the proof that the
+ * likewise for the Hadamard kernel's division by sqrt(32) and sqrt(128), its one-multiplication form on
+ * every 16-bit pattern, and the fp32 inputs' division by a tensor scale), and the proof that the
  * E2M1 rounding done on the FP4 conversion unit equals the reference's round-half-up
  * (project_quant/codebook.py:12-25) for every fp32 magnitude from 0 to 16, level and code;
  * it leaves the number of disagreements (expected 0) in *mismatches (device memory). */
@@ -317,8 +318,8 @@ MIXFP4_API int mixfp4_gemv_allreduce(const mixfp4_comm* comm, const void* x, int
 MIXFP4_API int mixfp4_set_wait_limit_ns(uint64_t ns);
 MIXFP4_API int mixfp4_check_status(const int* dev_status, int* value, void* stream);
 
-/* Prefill-shape dequant-linear on the tcgen05 tensor cores (any M >= 1, meant for
- * M >= 128).  rotation_block: 0, or 128 to apply the block-Hadamard H128 to x first (the
+/* Dequant-linear on the tcgen05 tensor cores (any M >= 1; up to 128 rows of the kernel and stream layouts run
+ * a kernel of their own that needs no partial sums and takes MIXFP4_FLAG_OVERLAP_PREVIOUS).  rotation_block: 0, or 128 to apply the block-Hadamard H128 to x first (the
  * reference's forward-pre-hook, modeling.py:662-668): a rotation kernel of its own writes
  * bf16(FWHT_fp32(x)) into the workspace and the GEMM kernel, launched behind it as a programmatic
  * dependent, reads that (its set-up and weight loads overlap the rotation's tail; the rotation is

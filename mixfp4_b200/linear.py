@@ -3,9 +3,9 @@ reference would have overwritten with its dequantized tensor
 (project_quant/modeling.py:603-639 quantize_model_weights, :629 the weight swap, and the
 activation rotation pre-hook :662-668).
 
-``mixfp4_linear`` picks the kernel by shape alone: M <= 16 runs the HBM-bound GEMV,
-larger M the tcgen05 GEMM.  There is one implementation per shape class and no
-fallback.
+``mixfp4_linear`` picks the kernel by shape alone: M <= 16 runs the HBM-bound GEMV, up to 128
+rows the kernel that decodes the weight into tensor memory, larger M the tcgen05 GEMM.  There is one
+implementation per shape class and no fallback.
 """
 
 from __future__ import annotations
@@ -79,7 +79,7 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
     its own into the workspace and starts the GEMM kernel under that pass's tail; the GEMV path
     and other block sizes call the FWHT kernel here (fp32 stages, one rounding, in both cases).
     out_dtype: torch.float32 or torch.bfloat16 (default: x.dtype).
-    overlap_previous: launch the decode kernel as a programmatic dependent of the previous
+    overlap_previous: launch the kernel (up to 128 rows of x) as a programmatic dependent of the previous
     kernel in the stream (its weight prefetch overlaps that kernel's tail).  Only valid when
     the previous kernel does not write this layer's packed weight.
     """
