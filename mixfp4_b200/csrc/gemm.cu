@@ -906,6 +906,8 @@ int launch_gemm_pair(const void* xa, int64_t lda, const GemmArgs& args, cudaStre
 
 using namespace mixfp4;
 
+int64_t mixfp4::gemm_tile_chain(int64_t m, int64_t n, int64_t k) { return (int64_t)plan_gemm(m, n, k).kt_per_split * BK; }
+
 // Argument checks shared by every GEMM entry point; they run before anything is enqueued.
 static int check_gemm_args(const void* x, int64_t m, int64_t ldx, const uint8_t* codes, const uint8_t* scales,
                            const uint8_t* fmt, const float* global_scale, int64_t n, int64_t k, int layout,
@@ -968,7 +970,8 @@ static int gemm_run(const void* x, int64_t m, int64_t ldx, const uint8_t* codes,
     if (layout != MIXFP4_LAYOUT_CANONICAL && m <= kSmallMaxTokens) {
         const mixfp4_gemv_segment seg = {codes, scales, global_scale, lut, y, ldy, n};
         const bool dependent = rotation_block == 128 || ((x_from_previous_kernel || overlap_previous) && xa == x);
-        const int rc = gemm_small(xa, m, lda, k, &seg, 1, layout == MIXFP4_LAYOUT_STREAM, out_dtype, dependent, status, st);
+        const int rc = gemm_small(xa, m, lda, k, &seg, 1, layout == MIXFP4_LAYOUT_STREAM, out_dtype, gemm_tile_chain(m, n, k),
+                                  dependent, status, st);
         if (rc != MIXFP4_E_SHAPE) return rc;         // sizes beyond its index range: the tiles below
     }
 

@@ -79,7 +79,9 @@ struct SmallArgs {
     int d_cols;                                     // TMEM columns of an accumulator: np rounded up to 32
     int chains;                                     // accumulators per piece (1, 2 or 4), units in turn: see gemm_small
     int slots;                                      // sums of cut tiles kept apart from the rings: 0, 1 or 2
-    int flush;                                      // 0, or units after which a piece's accumulators are added up in registers
+    uint32_t part[2];                               // where they are in the end: a run's first piece, its last one behind others
+    int flush;                                      // 0, or units after which a piece's accumulators are added to its sums
+    int sum_cols;                                   // flush with more than 16 tokens: TMEM columns of the sums (16: registers)
     int sets;                                       // sets of accumulators: 3, or 2 when no piece has to stay in TMEM
     int a_stages;                                   // A stages (units, with their x): 4, or 2 when the accumulators need the columns
     int x_pair;                                     // x comes in boxes of 2 x 64 K (K a multiple of 64), else one by one
@@ -174,6 +176,18 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(v[i]);
+}
+// thread i of the warp writes lane base+i, 16 columns (no wait: tcgen05.wait::st before they are read)
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const float (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::"r"(__float_as_uint(r[0])), "r"(__float_as_uint(r[1])), "r"(__float_as_uint(r[2])), "r"(__float_as_uint(r[3])),
+          "r"(__float_as_uint(r[4])), "r"(__float_as_uint(r[5])), "r"(__float_as_uint(r[6])), "r"(__float_as_uint(r[7])),
+          "r"(__float_as_uint(r[8])), "r"(__float_as_uint(r[9])), "r"(__float_as_uint(r[10])), "r"(__float_as_uint(r[11])),
+          "r"(__float_as_uint(r[12])), "r"(__float_as_uint(r[13])), "r"(__float_as_uint(r[14])), "r"(__float_as_uint(r[15])),
+          "r"(taddr)
+        : "memory");
 }
 __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {      // the same offset in a CTA of the cluster
     uint32_t remote;
@@ -308,8 +322,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     else asm volatile("barrier.cta.sync 1, %0;" ::"n"(kThreadsS) : "memory");
     tcgen05_fence_after();
     const uint32_t tmem_base = warp < 2 ? 0u : __shfl_sync(0xffffffffu, *tmem_slot, 0);
-    const uint32_t d_cols = (uint32_t)a.d_cols;               // TMEM: three sets of accumulators | A stages
-    const uint32_t a_base = tmem_base + a.sets * a.chains * d_cols;
+    const uint32_t d_cols = (uint32_t)a.d_cols;               // TMEM: sets of accumulators | sums (flush) | A stages
+    const uint32_t sum_base = tmem_base + a.sets * a.chains * d_cols, a_base = sum_base + a.sum_cols;
     // accumulator set of a run's piece p and how often it has been used before: two sets in turn, or three, where the
     // first piece may be a cut tile that has to stay in its own
     auto d_of = [&](int p) { return a.sets == 2 ? p & 1 : p == 0 ? 0 : 1 + ((p - 1) & 1); };
@@ -429,7 +443,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         // epilogue of the tiles this run holds from end to end
         const int q = warp & 3, row = tile_row(q, lane);
         int set = 0, par = 0;
-        for (int p = 0; a.flush && p < npieces; ++p) {              // 16 tokens at most: the sums fit in registers
+        for (int p = 0; a.flush && a.sum_cols == 0 && p < npieces; ++p) {   // 16 tokens at most: the sums fit in registers
             float sum[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) sum[j] = 0.0f;
@@ -461,10 +475,61 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                     for (int j = 0; j < 16; ++j)
                         if (j < a.m) store_y(seg, a.out_dtype, j, n0, sum[j]);
             } else {
-                float* part = reinterpret_cast<float*>(gen + L.parts) + (p == 0 ? 0 : np * kTileRows) + q * 32 + lane;
+                float* part = reinterpret_cast<float*>(gen + a.part[p > 0]) + q * 32 + lane;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) part[j * kTileRows] = sum[j];
             }
+        }
+        // more tokens: the sums of a piece longer than the flush interval lie in TMEM between its parts
+        for (int p = 0; a.sum_cols && p < npieces; ++p) {
+            const bool whole = piece_whole(p);
+            const int tile = t0 + tile_first + p, sg = seg_of(tile);
+            const SmallSegment& seg = a.seg[sg];
+            const int n0 = (tile - seg_first(sg)) * kTileRows + row;
+            float* part = reinterpret_cast<float*>(gen + a.part[p > 0]) + q * 32 + lane;
+            const bool stays = !whole && a.part[p > 0] == 0;        // goes where the rings are: in TMEM until they are free
+            const uint32_t lanes = (uint32_t)(q * 32) << 16;
+            const int lo = (tile_first + p) * S;
+            bool ok = true, first = true;
+            for (int len = min(lo + S, ub) - max(lo, ua); len > 0 && ok; len -= a.flush) {
+                ok = warp_wait(full_d(set), par, ctx, 6);
+                if (!ok) break;
+                tcgen05_fence_after();
+                const bool last = len <= a.flush;
+                for (int c = 0; c < np; c += 16) {
+                    float v[16];
+                    tmem_ld_32x16(tmem_base + lanes + (uint32_t)(set * a.chains) * d_cols + c, v);
+                    for (int i = 1; i < min(a.chains, len); ++i) {
+                        float w[16];
+                        tmem_ld_32x16(tmem_base + lanes + (uint32_t)(set * a.chains + i) * d_cols + c, w);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += w[j];
+                    }
+                    if (!first) {
+                        float w[16];
+                        tmem_ld_32x16(sum_base + lanes + c, w);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += w[j];
+                    }
+                    if (!last || stays) {
+                        tmem_st_32x16(sum_base + lanes + c, v);
+                    } else if (!whole) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) part[(c + j) * kTileRows] = v[j];
+                    } else if (n0 < seg.n) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (c + j < a.m) store_y(seg, a.out_dtype, c + j, n0, v[j]);
+                    }
+                }
+                if (!last || stays) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                first = false;
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty_d(set));
+                if (++set == a.sets) { set = 0; par ^= 1; }
+            }
+            if (!ok) break;
         }
         for (int p = 0; !a.flush && p < npieces; ++p) {
             const int d = d_of(p);
@@ -479,7 +544,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                 float v[16];
                 load_piece(p, c, v);
                 if (!whole) {                                       // a cluster of two: one cut tile per run
-                    float* part = reinterpret_cast<float*>(gen + L.parts) + c * kTileRows + q * 32 + lane;
+                    float* part = reinterpret_cast<float*>(gen + a.part[p > 0]) + c * kTileRows + q * 32 + lane;
 #pragma unroll
                     for (int j = 0; j < 16; ++j) part[j * kTileRows] = v[j];
                 } else if (n0 < seg.n) {
@@ -562,23 +627,22 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
 
     if (a.cluster > 1) {
         // Tiles cut by run boundaries.  All copies have landed and all MMAs are done (the epilogue warps have waited
-        // for every piece), so the rings are free: [first piece, last piece][token][TMEM lane] fp32.
+        // for every piece), so the rings are free: [token][TMEM lane] fp32 at part[0] (first piece) and part[1] (last).
         // (Sums that have slots are there already.)
-        const uint32_t parts_at = a.slots ? L.parts : 0u;
-        float* parts = reinterpret_cast<float*>(gen + parts_at);
-        const uint32_t part_stride = (uint32_t)np * kTileRows;
         const int tl_index = (warp & 3) * 32 + lane;
         __syncthreads();
-        if (a.slots == 0 && warp >= 4 && warp < 8) {
+        if ((a.slots == 0 || a.part[1] == 0) && warp >= 4 && warp < 8) {
             tcgen05_fence_after();
-            for (int i = 0; i < 2; ++i) {
+            for (int i = a.slots; i < 2; ++i) {
                 const int p = i == 0 ? 0 : npieces - 1;
                 if ((i == 1 && npieces == 1) || piece_whole(p)) continue;
+                float* part = reinterpret_cast<float*>(gen + a.part[i]) + tl_index;
                 for (int c = 0; c < np; c += 16) {
                     float v[16];
-                    load_piece(p, c, v);
+                    if (a.sum_cols) tmem_ld_32x16(sum_base + ((uint32_t)((warp & 3) * 32) << 16) + c, v);
+                    else load_piece(p, c, v);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) parts[i * part_stride + (c + j) * kTileRows + tl_index] = v[j];
+                    for (int j = 0; j < 16; ++j) part[(c + j) * kTileRows] = v[j];
                 }
             }
         }
@@ -596,7 +660,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
 #pragma unroll
             for (int w2 = 0; w2 < kMaxCluster; ++w2)
                 if (w2 < share)
-                    src[w2] = peer_addr(base + parts_at + (uint32_t)lane * 16u + (w2 == 0 && (packed >> 16) && a.slots != 1 ? part_stride * 4u : 0u), (uint32_t)(wf + w2));
+                    src[w2] = peer_addr(base + (uint32_t)lane * 16u + a.part[w2 == 0 && (packed >> 16)], (uint32_t)(wf + w2));
             for (int b = (rank - wf) + share * warp; b < a.m; b += share * (kThreadsS / 32)) {
                 float4 v[kMaxCluster];
 #pragma unroll
@@ -628,6 +692,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
 
 // ------------------------------------------------------------------------- host side
 constexpr uint32_t kSmemLimitS = 227 * 1024;
+// accumulators per piece where nothing is flushed (three sets of them beside the A stages in 512 TMEM columns)
+int small_chains(int np) { return np <= 32 ? 4 : np <= 64 ? 2 : 1; }
 constexpr int kMaxDevicesS = 64;
 
 // How many clusters of each size the current device runs at once (one CTA per SM), asked once per device.
@@ -676,21 +742,29 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
 // gemm_kernel (seven launches and up to seven split-K sums a layer), 508 us with four launches of this kernel.  Launches
 // alone, 48 tokens: 4096 x 4096 8.7 us, 6144 x 4096 in three weights 10.6 us, 28672 x 4096 in two 27.9 us, 4096 x 14336
 // 17.3 us.  The decode's byte permutes keep the ALU busy for 476 cycles of a unit.
-SmallPlan plan_small(int ntiles, int units, const int* clusters) {
-    SmallPlan best = {0, 0};
+//
+// chain_limit (products, a multiple of 128): a chain of the tensor core's accumulation is no longer than that.  The longest
+// piece of a run is cut by the accumulators it has in turn; where that is not enough its accumulators are flushed
+// into sums in TMEM (error against fp64 and time, 128 tokens, without the limit and with it: 4096 x 4096 1.72e-6 -> 7.8e-7,
+// 15.0 -> 15.7 us; 8192 x 28672 9.2e-6 -> 4.0e-6, 73.5 -> 73.8 us; 12288 x 14336 9.4e-6 -> 4.4e-6, 45.7 -> 46.5 us).
+SmallPlan plan_small(int ntiles, int units, int np, int64_t chain_limit, const int* clusters) {
+    SmallPlan best = {0, 0, 0};
     double t_best = 1e300;
+    const int chains = small_chains(np), limit = chain_limit > kUnitK ? (int)(chain_limit / kUnitK) : 1;
     for (int c = 1; c <= kMaxCluster && c <= units; c += c == 1 ? 1 : 2) {
         if (clusters[c] < 1) continue;
         const int n = ntiles < clusters[c] ? ntiles : clusters[c];
         const int64_t longest = ((int64_t)((ntiles + n - 1) / n) * units + c - 1) / c;
+        const int piece = (int)(longest < units ? longest : units);
+        const bool flush = np > 16 && (piece + chains - 1) / chains > limit;
         const double t = (double)longest + (c == 1 ? 0.0 : c == 2 ? 1.0 : 9.0);
-        if (t < t_best) { t_best = t; best.cluster = c; best.nclusters = n; }
+        if (t < t_best) { t_best = t; best.cluster = c; best.nclusters = n; best.flush = flush ? limit : 0; }
     }
     return best;
 }
 
 int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_gemv_segment* segments, int count,
-               bool stream_layout, int out_dtype, bool dependent, int* status, cudaStream_t st) {
+               bool stream_layout, int out_dtype, int64_t chain_limit, bool dependent, int* status, cudaStream_t st) {
     if (m < 1 || m > (count > 1 ? kSmallMaxGrouped : kSmallMaxTokens) || count < 1 || count > kMaxSegS) return MIXFP4_E_SHAPE;
     if (!aligned(x, 16) || ldx % 8 != 0) return MIXFP4_E_ALIGN;
     EncodeTiledFn encode = encode_tiled_fn();
@@ -748,7 +822,7 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
     }
     int clusters[kMaxCluster + 1];
     if (const int rc = max_clusters(clusters)) return rc;
-    const SmallPlan plan = plan_small((int)tiles, a.units, clusters);
+    const SmallPlan plan = plan_small((int)tiles, a.units, a.np, chain_limit, clusters);
     if (plan.cluster < 1) return MIXFP4_E_UNSUPPORTED;
     a.cluster = plan.cluster;
     a.per_cluster = (int)tiles / plan.nclusters;
@@ -758,20 +832,23 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
     a.split_more = RunSplit{n1 / a.cluster, n1 % a.cluster};
     a.inv_cluster = 65536u / (uint32_t)a.cluster + 1;
     a.inv_units = a.units == 1 ? 0xffffffffu : (uint32_t)((1ull << 32) / (uint32_t)a.units);
-    // TMEM (512 columns): two or three sets of accumulators, 4 or 2 A stages of 64 columns.  The tensor core's accumulation
-    // error grows with the number of products in a chain (3.7e-6 of the result after 4096, 8e-7 after 1024, against
-    // fp64), so a piece's units go to as many accumulators in turn as there is room for and the sums are added in fp32.
+    // TMEM (512 columns): two or three sets of accumulators, the sums of flushed ones, 4 or 2 A stages of 64 columns.  The
+    // tensor core's accumulation error grows with the number of products in a chain (7.8e-7 of the result after 1024, 1.7e-6
+    // after 2048, 3.6e-6 after 4096, 9.3e-6 after 14336 against fp64), so a piece's units go to as many accumulators in turn
+    // as there is room for and the sums are added in fp32.
     a.d_cols = (a.np + 31) / 32 * 32;
-    a.chains = a.d_cols <= 32 ? 4 : a.d_cols <= 64 ? 2 : 1;
+    a.chains = plan.flush ? 1 : small_chains(a.np);
     // Up to 16 tokens stand in for matrix-vector kernels that split K finely: chains of 256 products at most, added up in
-    // the epilogue warps' registers.
-    a.flush = a.np == 16 ? 2 * a.chains : 0;
+    // the epilogue warps' registers.  More tokens whose pieces exceed the limit: added up in TMEM.
+    a.flush = a.np == 16 ? 2 * a.chains : plan.flush;
+    a.sum_cols = plan.flush ? a.d_cols : 0;
     // A run has a cut tile at each end at most, in a cluster of two only at one; sums that leave TMEM as soon as their
     // piece is complete free a set of accumulators for two more A stages (28672 x 4096, 48 tokens: about a tenth).
-    // (Beyond 64 tokens shared memory has no room for them.)
-    a.slots = a.cluster == 1 || a.np > 64 ? 0 : a.flush ? 2 : a.cluster == 2 ? 1 : 0;
-    a.sets = a.np <= 64 && (a.cluster <= 2 || a.flush) ? 2 : 3;
-    a.a_stages = a.sets * a.chains * a.d_cols + 4 * 64 <= (int)kTmemColsS ? 4 : 2;
+    // (Beyond 64 tokens shared memory has room for one slot, which only flushing needs: a first piece's sums would be in the
+    // way of the next one's; the last piece's stay in TMEM.)
+    a.slots = a.cluster == 1 ? 0 : a.flush ? (a.np <= 64 ? 2 : 1) : a.cluster == 2 && a.np <= 64 ? 1 : 0;
+    a.sets = a.flush || (a.np <= 64 && a.cluster <= 2) ? 2 : 3;
+    a.a_stages = a.sets * a.chains * a.d_cols + a.sum_cols + 4 * 64 <= (int)kTmemColsS ? 4 : 2;
     // shared memory: eight weight stages and eight copies of the tables where they fit
     const int choices[6][2] = {{8, 3}, {8, 2}, {4, 3}, {4, 2}, {4, 1}, {4, 0}};
     for (const auto& c : choices) {
@@ -780,8 +857,11 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
         if (small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.slots).bytes <= kSmemLimitS) break;
     }
     const SmallLayout L = small_layout(a.np, count, a.w_stages, a.a_stages, a.lut_shift, a.slots);
-    // (the partial sums of cut tiles, 2 * np * 512 bytes, go where the rings were)
-    if (L.bytes > kSmemLimitS || (a.slots == 0 && (uint32_t)a.np * kTileRows * 8u > L.lut)) return MIXFP4_E_SHAPE;
+    const uint32_t part_bytes = (uint32_t)a.np * kTileRows * 4u;
+    a.part[0] = a.slots ? L.parts : 0u;
+    a.part[1] = a.slots != 1 ? a.part[0] + part_bytes : a.cluster == 2 ? a.part[0] : 0u;
+    // (sums of cut tiles without a slot go where the rings were)
+    if (L.bytes > kSmemLimitS || (2 - a.slots) * part_bytes > L.lut) return MIXFP4_E_SHAPE;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(plan.cluster * plan.nclusters));
     cfg.blockDim = dim3(kThreadsS);
@@ -817,6 +897,11 @@ extern "C" int mixfp4_gemm_grouped(const void* x, int64_t m, int64_t ldx, int64_
         if (in.n <= 0 || in.n > 0x7fffffffLL || in.ldy < in.n) return MIXFP4_E_SHAPE;
         if (!aligned(in.codes, 16) || (in.lut && !aligned(in.lut, 16))) return MIXFP4_E_ALIGN;
     }
-    return gemm_small(x, m, ldx, k, segments, count, true, out_dtype, (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0, status,
+    int64_t chain = INT64_MAX;
+    for (int s = 0; s < count; ++s) {
+        const int64_t c = gemm_tile_chain(m, segments[s].n, k);
+        chain = c < chain ? c : chain;
+    }
+    return gemm_small(x, m, ldx, k, segments, count, true, out_dtype, chain, (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0, status,
                       static_cast<cudaStream_t>(stream));
 }

@@ -130,3 +130,40 @@ def test_grouped_entry_checks_its_arguments():
     assert call() == nat.E_ALIGN
     seg[0].codes, seg[0].y = 16, None
     assert call() == nat.E_NULL
+
+
+def gpu_weight(n, k, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return mx.quantize_packed((torch.randn((n, k), generator=gen, device="cuda") * 0.02).to(torch.bfloat16))[0]
+
+
+def errors(y, ref):
+    """Error of the whole result and of its worst 128 columns (a tile of the kernel), relative 2-norms."""
+    diff = y.double() - ref
+    whole = (diff.norm() / ref.norm()).item()
+    tiles = [(diff[:, c:c + 128].norm() / ref[:, c:c + 128].norm()).item() for c in range(0, ref.shape[1], 128)]
+    return whole, max(tiles)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,ns,k", [
+    (65, (2048,), 2048), (65, (4096,), 4096), (96, (4096,), 4096), (128, (4096,), 4096), (100, (6144,), 4096),
+    (65, (8192,), 8192), (72, (3000,), 8192), (65, (4096,), 14336), (128, (4096,), 14336), (80, (12288,), 14336),
+    (128, (12288,), 14336), (65, (8192,), 28672), (96, (8192,), 28672), (128, (8192,), 28672), (48, (12288,), 14336),
+    (17, (4096, 1024, 1024), 4096), (48, (4096, 1024, 1024), 4096), (32, (8192, 1024, 1024), 8192),
+    (64, (8192, 1024, 1024), 8192), (33, (300, 17), 1112)])
+def test_error_is_that_of_the_tiles(m, ns, k):
+    """The tensor core's accumulation error grows in proportion to the products summed in one accumulator (after 1024: 7.8e-7
+    of the result, after 2048: 1.7e-6), so no accumulator may sum more of them than one of the 128-row tiles that the same
+    weight in the canonical layout runs on.  With chains as long the errors agree up to their scatter (2 percent over at least
+    17 x 128 outputs; 0.2 of 2^-23 is allowed for the additions of partial sums, whose number differs); a chain twice as
+    long doubles the error."""
+    packs = [gpu_weight(n, k, n + k + i) for i, n in enumerate(ns)]
+    x = synth.activations(m, k, m).cuda()
+    ys = mx.mixfp4_linear_grouped(x, [p.to_stream_layout() for p in packs], out_dtype=torch.float32)
+    for y, p in zip(ys, packs):
+        ref = x.double() @ p.dequantize().double().T
+        got, tiles = errors(y, ref), errors(mx.mixfp4_linear(x, p, out_dtype=torch.float32), ref)
+        assert all(g <= 1.15 * t + 0.2 * 2.0 ** -23 for g, t in zip(got, tiles))
+        assert torch.equal(mx.mixfp4_linear(x, p.to_kernel_layout()), mx.mixfp4_linear(x, p.to_stream_layout()))
+    assert mx.gemm_status() == 0
