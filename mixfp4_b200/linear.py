@@ -246,7 +246,7 @@ class MixFP4Linear(nn.Module):
             w = w.to(torch.bfloat16)
         amax = None
         if rotation is not None:
-            amax = torch.empty(1, dtype=torch.float32, device=device)
+            amax = torch.empty(1, dtype=torch.float32, device=w.device)
             rotated = _rotation.apply_transform(w, rotation, amax=amax)
             w, amax = rotated, (amax if rotated is not w else None)
         if mode in _MODE_CODE:

@@ -117,7 +117,11 @@ def apply_transform(x: torch.Tensor, value: str | TransformSpec, *, rounding: st
         return x
     if size not in _SUPPORTED_SIZES:
         raise NotImplementedError(f"the FWHT kernel supports block sizes {_SUPPORTED_SIZES}, got {size}")
+    if amax is not None:
+        nat.require_cuda(amax, "amax")              # a kernel writes to it
     dev = x.device if x.is_cuda else torch.device("cuda", torch.cuda.current_device())
+    if amax is not None and (amax.device != dev or amax.dtype != torch.float32 or amax.numel() < 1):
+        raise ValueError("amax must be a float32 tensor on the transform's device")
     signs = _device_signs(size, spec.seed, dev) if spec.seed is not None else None
     return _run_fwht(x, size, signs, stagewise=(rounding == "reference"), amax=amax)
 

@@ -205,3 +205,13 @@ def test_activation_modes_follow_the_reference_tables():
     assert quant.region_shape("m16k16", "activation_a") == (16, 1)
     assert quant.region_shape("n8k16", "weight_b") == (8, 1)
     assert quant.region_shape("layer", "weight_b") == quant.region_shape("layer", "activation_a") == (1, 0)
+
+
+@pytest.mark.parametrize("rotation", ["H128", "H16", "random_signed_H64_seed0"])
+def test_host_weights_and_host_amax_are_refused_before_any_kernel(rotation):
+    """A kernel writes the maximum through the pointer it is given: a host tensor there must never reach it."""
+    linear = torch.nn.Linear(256, 32, bias=False, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="must be a CUDA tensor"):
+        mx.MixFP4Linear.from_linear(linear, rotation=rotation, device="cpu")
+    with pytest.raises(RuntimeError, match="amax must be a CUDA tensor"):
+        mx.apply_transform(torch.zeros(4, 256), rotation, amax=torch.zeros(1))
