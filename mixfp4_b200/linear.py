@@ -92,7 +92,8 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
     if out_dtype not in (torch.float32, torch.bfloat16):
         raise TypeError("out_dtype must be float32 or bfloat16")
     lead = x.shape[:-1]
-    x2 = x if x.dim() == 2 else x.reshape(-1, packed.k)
+    # a view only where it changes something: more dimensions, or a single row, whose stride can be any number
+    x2 = x if x.dim() == 2 and (x.shape[0] > 1 or x.stride(0) == packed.k) else x.reshape(-1, packed.k)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     m = x2.shape[0]

@@ -93,3 +93,20 @@ def test_gemv_property_linearity_full_size():
     wq = oracle.bf16_bits_to_f32(oracle.dequant(oracle.quantize(w.float().numpy()), "bf16"))
     ystar = oracle.linear(x1.float().numpy(), wq[rows])
     assert oracle.relative_l2(f(x1)[:, rows].numpy(), ystar) <= TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["canonical", "kernel", "stream"])
+def test_a_single_row_with_any_stride(layout):
+    """[1, K] views whose row stride is no row length: a transposed column, a row of a wider array, an expanded vector."""
+    k = 264
+    packed = mx.quantize_packed(synth.student_t_weight(40, k, 7).cuda(), rotation="H128")[0]
+    packed = {"canonical": packed.to_canonical, "kernel": packed.to_kernel_layout, "stream": packed.to_stream_layout}[layout]()
+    row = synth.activations(1, k, 3).cuda()
+    wide = torch.zeros((3, k + 3), dtype=torch.bfloat16, device="cuda")
+    wide[1, :k] = row[0]
+    for kwargs in ({}, {"rotate": False}, {"activation_mode": "oracle16"}):
+        want = mx.mixfp4_linear(row, packed, **kwargs)
+        for view in (row.reshape(k, 1).T, wide[1:2, :k], row[0].expand(1, k), row.as_strided((1, k), (0, 1)), row.as_strided((1, k), (8, 1))):
+            assert view.shape == (1, k)
+            assert torch.equal(mx.mixfp4_linear(view, packed, **kwargs), want)
