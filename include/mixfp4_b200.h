@@ -340,7 +340,8 @@ MIXFP4_API int mixfp4_gemm(const void* x, int64_t m, int64_t ldx,
 
 /* mixfp4_gemv_grouped's counterpart for a batch of tokens: up to three stream-layout weights that share x in
  * one launch, 1 <= M <= 64, x with 16-byte aligned rows (MIXFP4_E_ALIGN otherwise: call mixfp4_gemm per weight).
- * status as in mixfp4_gemm; flags: MIXFP4_FLAG_OVERLAP_PREVIOUS. */
+ * status as in mixfp4_gemm, but with M <= 16 and NULL the decode kernels' own word (mixfp4_check_status); waits are
+ * limited as theirs with M <= 16 (mixfp4_set_wait_limit_ns), else as mixfp4_gemm's.  flags: MIXFP4_FLAG_OVERLAP_PREVIOUS. */
 MIXFP4_API int mixfp4_gemm_grouped(const void* x, int64_t m, int64_t ldx, int64_t k,
                         const mixfp4_gemv_segment* segments, int count, int layout, int out_dtype,
                         int* status, int flags, void* stream);

@@ -971,7 +971,7 @@ static int gemm_run(const void* x, int64_t m, int64_t ldx, const uint8_t* codes,
         const mixfp4_gemv_segment seg = {codes, scales, global_scale, lut, y, ldy, n};
         const bool dependent = rotation_block == 128 || ((x_from_previous_kernel || overlap_previous) && xa == x);
         const int rc = gemm_small(xa, m, lda, k, &seg, 1, layout == MIXFP4_LAYOUT_STREAM, out_dtype, gemm_tile_chain(m, n, k),
-                                  dependent, status, st);
+                                  kWaitLimitNs, dependent, status, st);
         if (rc != MIXFP4_E_SHAPE) return rc;         // sizes beyond its index range: the tiles below
     }
 

@@ -40,6 +40,7 @@
 #include "common.cuh"
 #include "decode.cuh"
 #include "gemm_small.cuh"
+#include "gemv_common.cuh"
 #include "tcgen05.cuh"
 
 namespace mixfp4 {
@@ -87,6 +88,7 @@ struct SmallArgs {
     int x_pair;                                     // x comes in boxes of 2 x 64 K (K a multiple of 64), else one by one
     int w_stages, lut_shift;                        // weight stages (a power of two); 2^lut_shift copies of the decode table
     int* status;
+    uint64_t wait_ns;                               // limit of a wait
 };
 struct SmallMaps {
     CUtensorMap x;
@@ -199,6 +201,9 @@ __device__ __forceinline__ float4 ld_peer_f32x4(uint32_t remote) {
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
     return v;
 }
+// End of the kernel before (nothing to wait for without a dependent launch).  Every role comes here before the first wait
+// that x can hold up, so that the time limit of its waits does not run while that kernel does.
+__device__ __forceinline__ void wait_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Wait of a whole warp: the vote makes the result (and what is computed from it) provably uniform, so the loops of
 // the single-warp roles run on the uniform datapath, where TMA and MMA instructions take their operands from.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int code) {
@@ -254,7 +259,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L.misc);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L.misc + 4);
     volatile int* sharer = reinterpret_cast<volatile int*>(gen + L.misc + 16);     // first and last CTA of the run's cut tiles
-    const WaitCtx ctx{abort_flag, a.status};
+    const WaitCtx ctx{abort_flag, a.status, a.wait_ns};
 
     // The next kernel in the stream may set itself up from here on; it waits for this grid's end before it
     // reads this one's outputs.
@@ -358,6 +363,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         uint32_t parity = 1;                                        // of the stage's last release
         while (w_issued < cnt && ok) {
             if (w_stage == 0 && w_issued > 0) parity ^= 1;
+            if (w_issued == a.w_stages) wait_previous_grid();
             if (w_issued >= a.w_stages) ok = warp_wait(empty_w(w_stage), parity, ctx, 7);
             if (ok) load_w();
         }
@@ -365,7 +371,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         for (int u = max(0, w_issued - a.w_stages); u < w_issued && ok; ++u) ok = warp_wait(full_w(u & w_mask), (u / a.w_stages) & 1, ctx, 8);
     } else if (warp == 1) {
         // x (and nothing else this kernel reads) may come from the kernel launched just before
-        asm volatile("griddepcontrol.wait;" ::: "memory");
+        wait_previous_grid();
         asm volatile("fence.proxy.async.global;" ::: "memory");
         const uint32_t box = (uint32_t)np * 128u;
         int sub = sub_first;
@@ -397,6 +403,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         int piece = 0, done = 0, left = min(S - sub_first, cnt);    // units of the piece done (since the last flush) and left
         int set = 0, set_par = 1;                                   // flushing: sets in turn
         bool ok = true;
+        wait_previous_grid();
         for (int u = 0; u < cnt; ++u) {
             ok = warp_wait(full_a(u & 3), (u >> 2) & 1, ctx, 4);
             if (!ok) break;
@@ -443,6 +450,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         // epilogue of the tiles this run holds from end to end
         const int q = warp & 3, row = tile_row(q, lane);
         int set = 0, par = 0;
+        wait_previous_grid();
         for (int p = 0; a.flush && a.sum_cols == 0 && p < npieces; ++p) {   // 16 tokens at most: the sums fit in registers
             float sum[16];
 #pragma unroll
@@ -606,6 +614,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                     for (int j = 0; j < 4; ++j) { out[8 * b + j] = p0[j]; out[8 * b + 4 + j] = p1[j]; }
                 }
                 if (h == 0) {
+                    if (u >= a.a_stages && u < a.a_stages + kGroups) wait_previous_grid();
                     ok = wait_stage(u);
                     if (!ok) break;
                     tcgen05_fence_after();                          // the MMAs that read this stage are done
@@ -764,7 +773,8 @@ SmallPlan plan_small(int ntiles, int units, int np, int64_t chain_limit, const i
 }
 
 int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_gemv_segment* segments, int count,
-               bool stream_layout, int out_dtype, int64_t chain_limit, bool dependent, int* status, cudaStream_t st) {
+               bool stream_layout, int out_dtype, int64_t chain_limit, uint64_t wait_ns, bool dependent, int* status,
+               cudaStream_t st) {
     if (m < 1 || m > (count > 1 ? kSmallMaxGrouped : kSmallMaxTokens) || count < 1 || count > kMaxSegS) return MIXFP4_E_SHAPE;
     if (!aligned(x, 16) || ldx % 8 != 0) return MIXFP4_E_ALIGN;
     EncodeTiledFn encode = encode_tiled_fn();
@@ -777,6 +787,7 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
     a.nseg = count;
     a.out_dtype = out_dtype;
     a.status = status;
+    a.wait_ns = wait_ns;
     const int64_t units = padded_k(k) / kUnitK;
     const cuuint32_t estr[3] = {1, 1, 1};
     int64_t tiles = 0;
@@ -897,11 +908,15 @@ extern "C" int mixfp4_gemm_grouped(const void* x, int64_t m, int64_t ldx, int64_
         if (in.n <= 0 || in.n > 0x7fffffffLL || in.ldy < in.n) return MIXFP4_E_SHAPE;
         if (!aligned(in.codes, 16) || (in.lut && !aligned(in.lut, 16))) return MIXFP4_E_ALIGN;
     }
+    const bool decode = m <= 16;                       // rows that the decode kernels take: their wait limit, their status word
+    if (decode && !status) {
+        if (const int rc = stream_status_word(&status)) return rc;
+    }
     int64_t chain = INT64_MAX;
     for (int s = 0; s < count; ++s) {
         const int64_t c = gemm_tile_chain(m, segments[s].n, k);
         chain = c < chain ? c : chain;
     }
-    return gemm_small(x, m, ldx, k, segments, count, true, out_dtype, chain, (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0, status,
-                      static_cast<cudaStream_t>(stream));
+    return gemm_small(x, m, ldx, k, segments, count, true, out_dtype, chain, decode ? wait_limit_ns() : kWaitLimitNs,
+                      (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0, status, static_cast<cudaStream_t>(stream));
 }

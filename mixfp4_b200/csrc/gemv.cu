@@ -702,7 +702,8 @@ extern "C" int mixfp4_gemv(const void* x, int64_t m, int64_t ldx, const uint8_t*
         if (aligned(x, 16) && ldx % 8 == 0) {
             int* status = nullptr;
             if (const int rs = stream_status_word(&status)) return rs;
-            const int rg = gemm_small(x, m, ldx, k, &seg, 1, true, out_dtype, 256, (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0, status, st);
+            const int rg = gemm_small(x, m, ldx, k, &seg, 1, true, out_dtype, 256, wait_limit_ns(),
+                                      (flags & MIXFP4_FLAG_OVERLAP_PREVIOUS) != 0, status, st);
             if (rg != MIXFP4_E_SHAPE) return rg;
         }
     }

@@ -44,6 +44,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 struct WaitCtx {
     volatile int* abort_flag;   // shared memory
     int* status;                // global, may be null
+    uint64_t limit_ns = kWaitLimitNs;
 };
 
 // Bounded wait: false if the limit expired or another thread of the CTA already gave up.
@@ -55,7 +56,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const W
         if ((++spins & 63u) == 0) {
             if (*ctx.abort_flag) return false;
             // both a long time and many polls: a discontinuity of the timer alone never aborts a wait
-            if (spins > kMinSpins && global_timer_ns() - t0 > kWaitLimitNs) {
+            if (spins > kMinSpins && global_timer_ns() - t0 > ctx.limit_ns) {
                 *ctx.abort_flag = 1;
                 if (ctx.status) atomicCAS(ctx.status, 0, code);
                 return false;

@@ -207,7 +207,8 @@ def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dty
                 fn = "mixfp4_gemm_grouped"
                 st = nat.lib().mixfp4_gemm_grouped(x2.data_ptr(), m, x2.stride(0), k, segs, len(packs),
                                                    packs[0].layout_code, nat.DTYPE_CODE[out_dtype],
-                                                   _status_word(x.device).data_ptr(), flags, nat.stream_ptr(x.device))
+                                                   None if m <= GEMV_MAX_M else _status_word(x.device).data_ptr(),
+                                                   flags, nat.stream_ptr(x.device))    # None: the decode kernels' word
         if st != nat.E_SHAPE:
             nat.check(fn, st)
             return [y.reshape(*lead, p.n) for y, p in zip(ys, packs)]

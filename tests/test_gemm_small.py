@@ -167,3 +167,28 @@ def test_error_is_that_of_the_tiles(m, ns, k):
         assert all(g <= 1.15 * t + 0.2 * 2.0 ** -23 for g, t in zip(got, tiles))
         assert torch.equal(mx.mixfp4_linear(x, p.to_kernel_layout()), mx.mixfp4_linear(x, p.to_stream_layout()))
     assert mx.gemm_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,own", [(9, True), (16, True), (17, False), (64, False)])
+def test_decode_sizes_report_to_the_decode_kernels_word(monkeypatch, m, own):
+    """Rows that the decode kernels take (x too large for their shared memory) leave the status word to the library,
+    whose own one decode_status() reads; larger batches report to the GEMM's."""
+    k = 14336
+    packed, wd = weight(300, k, 5)
+    x = synth.activations(m, k, m).cuda()
+    lib, seen = nat.lib(), []
+
+    class Recorder:
+        def __getattr__(self, name):
+            fn = getattr(lib, name)
+            if name != "mixfp4_gemm_grouped":
+                return fn
+            return lambda *args: (seen.append(args[8]), fn(*args))[1]
+    monkeypatch.setattr(nat, "lib", lambda: Recorder())
+    ys = mx.mixfp4_linear_grouped(x, [packed, packed], out_dtype=torch.float32)
+    assert len(seen) == 1 and (seen[0] is None) == own
+    for y in ys:
+        check(y, x, wd, k, torch.float32)
+    monkeypatch.undo()
+    assert mx.decode_status() == 0 and mx.gemm_status() == 0
