@@ -204,6 +204,12 @@ __device__ __forceinline__ float4 ld_peer_f32x4(uint32_t remote) {
 // End of the kernel before (nothing to wait for without a dependent launch).  Every role comes here before the first wait
 // that x can hold up, so that the time limit of its waits does not run while that kernel does.
 __device__ __forceinline__ void wait_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A millisecond.
+__device__ __noinline__ void let_copies_land() {
+    const uint64_t t_0 = global_timer_ns();
+    while (global_timer_ns() - t_0 < 1000000ull) {}
+    __syncthreads();
+}
 // Wait of a whole warp: the vote makes the result (and what is computed from it) provably uniform, so the loops of
 // the single-warp roles run on the uniform datapath, where TMA and MMA instructions take their operands from.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int code) {
@@ -390,10 +396,6 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
             if (++sub == S) sub = 0;
         }
         // copies still in flight: the stages' MMAs wait for them, and the epilogue for the MMAs
-        if (!ok) {
-            const uint64_t t_0 = global_timer_ns();
-            while (global_timer_ns() - t_0 < 1000000ull) {}         // gave up: a last (bounded) chance for them to land
-        }
     } else if (warp == 2) {
         // kind::f16: D fp32, A and B bf16, both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(np >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -634,12 +636,18 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         }
     }
 
+    // Every role has stopped issuing.  Without an expired wait all copies have landed and all MMAs are done; after one, copies and
+    // MMAs may be in flight whoever gave up, and nothing tells when the last has ended (a role that stopped leaves barriers
+    // short of arrivals).  They get a millisecond, hundreds of times what a unit takes, before shared memory is written again,
+    // tensor memory is freed or the CTA leaves: a bounded wait, not a proof, and the status word is set by then.
+    tcgen05_fence_before();
+    __syncthreads();
+    if (*abort_flag) let_copies_land();              // (the same for all threads: nobody waits with a limit after the barrier)
     if (a.cluster > 1) {
-        // Tiles cut by run boundaries.  All copies have landed and all MMAs are done (the epilogue warps have waited
-        // for every piece), so the rings are free: [token][TMEM lane] fp32 at part[0] (first piece) and part[1] (last).
+        // Tiles cut by run boundaries.  The rings are free (the epilogue warps have waited for every piece's MMAs):
+        // [token][TMEM lane] fp32 at part[0] (first piece) and part[1] (last).
         // (Sums that have slots are there already.)
         const int tl_index = (warp & 3) * 32 + lane;
-        __syncthreads();
         if ((a.slots == 0 || a.part[1] == 0) && warp >= 4 && warp < 8) {
             tcgen05_fence_after();
             for (int i = a.slots; i < 2; ++i) {
@@ -687,10 +695,9 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         }
         __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        tcgen05_fence_before();
+        __syncthreads();
     }
-
-    tcgen05_fence_before();
-    __syncthreads();
     if (warp == 2) {
         tcgen05_fence_after();
         tmem_dealloc(tmem_base, kTmemColsS);
