@@ -221,8 +221,10 @@ __device__ __forceinline__ void store_y(const SmallSegment& s, int out_dtype, in
     else static_cast<__nv_bfloat16*>(s.y)[token * s.ldy + row] = __float2bfloat16_rn(v);
 }
 
-// kStream: the weights are in the stream layout, else in the kernel layout.
-template <bool kStream>
+// kStream: the weights are in the stream layout, else in the kernel layout.  kSums: pieces are flushed into sums in TMEM (a
+// kernel of its own: as one kernel the other form spilled; 28672 x 4096 at 48 tokens 26.9 us as one, 26.6 as two, 4096 x 4096
+// at 128 tokens 15.4 and 15.0).
+template <bool kStream, bool kSums>
 __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_constant__ SmallMaps maps,
                                                                   const __grid_constant__ SmallArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -453,7 +455,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         const int q = warp & 3, row = tile_row(q, lane);
         int set = 0, par = 0;
         wait_previous_grid();
-        for (int p = 0; a.flush && a.sum_cols == 0 && p < npieces; ++p) {   // 16 tokens at most: the sums fit in registers
+        for (int p = 0; !kSums && a.flush && p < npieces; ++p) {      // 16 tokens at most: the sums fit in registers
             float sum[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) sum[j] = 0.0f;
@@ -491,7 +493,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
             }
         }
         // more tokens: the sums of a piece longer than the flush interval lie in TMEM between its parts
-        for (int p = 0; a.sum_cols && p < npieces; ++p) {
+        for (int p = 0; kSums && p < npieces; ++p) {
             const bool whole = piece_whole(p);
             const int tile = t0 + tile_first + p, sg = seg_of(tile);
             const SmallSegment& seg = a.seg[sg];
@@ -506,15 +508,10 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                 if (!ok) break;
                 tcgen05_fence_after();
                 const bool last = len <= a.flush;
+#pragma unroll 1
                 for (int c = 0; c < np; c += 16) {
                     float v[16];
-                    tmem_ld_32x16(tmem_base + lanes + (uint32_t)(set * a.chains) * d_cols + c, v);
-                    for (int i = 1; i < min(a.chains, len); ++i) {
-                        float w[16];
-                        tmem_ld_32x16(tmem_base + lanes + (uint32_t)(set * a.chains + i) * d_cols + c, w);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] += w[j];
-                    }
+                    tmem_ld_32x16(tmem_base + lanes + (uint32_t)set * d_cols + c, v);
                     if (!first) {
                         float w[16];
                         tmem_ld_32x16(sum_base + lanes + c, w);
@@ -541,7 +538,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
             }
             if (!ok) break;
         }
-        for (int p = 0; !a.flush && p < npieces; ++p) {
+        for (int p = 0; !kSums && !a.flush && p < npieces; ++p) {
             const int d = d_of(p);
             if (!warp_wait(full_d(d), d_use(p) & 1, ctx, 6)) break;
             const bool whole = piece_whole(p);
@@ -648,15 +645,15 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         // [token][TMEM lane] fp32 at part[0] (first piece) and part[1] (last).
         // (Sums that have slots are there already.)
         const int tl_index = (warp & 3) * 32 + lane;
-        if ((a.slots == 0 || a.part[1] == 0) && warp >= 4 && warp < 8) {
+        if ((kSums ? a.part[1] == 0 : a.slots == 0) && warp >= 4 && warp < 8) {
             tcgen05_fence_after();
-            for (int i = a.slots; i < 2; ++i) {
+            for (int i = kSums ? 1 : 0; i < 2; ++i) {
                 const int p = i == 0 ? 0 : npieces - 1;
                 if ((i == 1 && npieces == 1) || piece_whole(p)) continue;
                 float* part = reinterpret_cast<float*>(gen + a.part[i]) + tl_index;
                 for (int c = 0; c < np; c += 16) {
                     float v[16];
-                    if (a.sum_cols) tmem_ld_32x16(sum_base + ((uint32_t)((warp & 3) * 32) << 16) + c, v);
+                    if (kSums) tmem_ld_32x16(sum_base + ((uint32_t)((warp & 3) * 32) << 16) + c, v);
                     else load_piece(p, c, v);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) part[(c + j) * kTileRows] = v[j];
@@ -722,8 +719,8 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
     if (dev < 0 || dev >= kMaxDevicesS) return MIXFP4_E_UNSUPPORTED;
     std::lock_guard<std::mutex> guard(lock);
     if (!have[dev]) {
-        MIXFP4_CUDA_CHECK(cudaFuncSetAttribute(gemm_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitS));
-        MIXFP4_CUDA_CHECK(cudaFuncSetAttribute(gemm_small_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitS));
+        for (const auto kernel : {gemm_small_kernel<true, false>, gemm_small_kernel<true, true>, gemm_small_kernel<false, false>, gemm_small_kernel<false, true>})
+            MIXFP4_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitS));
         for (int c = 1; c <= kMaxCluster; ++c) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)c);
@@ -736,7 +733,7 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, gemm_small_kernel<true>, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_small_kernel<true, false>, &cfg) != cudaSuccess) {
                 (void)cudaGetLastError();                    // a cluster size the device does not take
                 n = 0;
             }
@@ -762,7 +759,7 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
 // chain_limit (products, a multiple of 128): a chain of the tensor core's accumulation is no longer than that.  The longest
 // piece of a run is cut by the accumulators it has in turn; where that is not enough its accumulators are flushed
 // into sums in TMEM (error against fp64 and time, 128 tokens, without the limit and with it: 4096 x 4096 1.72e-6 -> 7.8e-7,
-// 15.0 -> 15.7 us; 8192 x 28672 9.2e-6 -> 4.0e-6, 73.5 -> 73.8 us; 12288 x 14336 9.4e-6 -> 4.4e-6, 45.7 -> 46.5 us).
+// 14.7 -> 15.0 us; 8192 x 28672 9.2e-6 -> 4.0e-6, 73.5 -> 73.8 us; 12288 x 14336 9.4e-6 -> 4.4e-6, 45.7 -> 46.5 us).
 SmallPlan plan_small(int ntiles, int units, int np, int64_t chain_limit, const int* clusters) {
     SmallPlan best = {0, 0, 0};
     double t_best = 1e300;
@@ -893,7 +890,9 @@ int gemm_small(const void* x, int64_t m, int64_t ldx, int64_t k, const mixfp4_ge
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = dependent ? 2 : 1;
-    MIXFP4_CUDA_CHECK(cudaLaunchKernelEx(&cfg, stream_layout ? gemm_small_kernel<true> : gemm_small_kernel<false>, maps, a));
+    const auto kernel = stream_layout ? (plan.flush ? gemm_small_kernel<true, true> : gemm_small_kernel<true, false>)
+                                      : (plan.flush ? gemm_small_kernel<false, true> : gemm_small_kernel<false, false>);
+    MIXFP4_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, maps, a));
     return check_launch("gemm_small_kernel");
 }
 
