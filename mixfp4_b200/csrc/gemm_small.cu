@@ -750,7 +750,13 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
 // Work split: the cluster size with the shortest longest run.  In units (about 0.37 us each), an exchange of partial
 // sums costs next to nothing between two CTAs and about nine units among four or more; odd sizes lose SMs and start
 // late (28672 x 4096, 48 tokens: 30.5, 30.3, 37.7, 31.4, 32.7, 31.6, 36.4, 33.0 us for 1 to 8 CTAs; 4096 x 14336: 44.5,
-// 24.3, 19.9, 17.4, 22.8, 18.0, 22.5, 20.4 us), and are left out.
+// 24.3, 19.9, 17.4, 22.8, 18.0, 22.5, 20.4 us), and are left out.  Nine is too much where every cluster has one tile:
+//   runs of at most 2048 K whose CTAs leave the next launch of a chain half of the SMs (2048 x 2048, 48 tokens, clusters of 2
+//   and 4: 10.3 and 8.7 us alone, 6.4 and 5.5 us in a chain; with more CTAs the chain loses, 4096 x 2048, 96 tokens: 7.7 and 9.1 us);
+//   more than 64 tokens, where clusters of two have two A stages as well (4096 x 4096, 128 tokens: 15.1 and 12.4 us alone, 12.8
+//   and 11.6 us in a chain);
+//   clusters of four on three quarters of the SMs (3000 x 4096, 17 tokens: 12.6 and 9.6 us alone, 8.4 and 8.1 us in a chain).
+// With nine there these took longer alone than the 128-row tiles (9.8 us for the first, 11.0 us for the last).
 // One decode step of 48 tokens through the linears of eight 8B-shaped decoder layers: 1358 us with the 128-row tiles of
 // gemm_kernel (seven launches and up to seven split-K sums a layer), 508 us with four launches of this kernel.  Launches
 // alone, 48 tokens: 4096 x 4096 8.7 us, 6144 x 4096 in three weights 10.6 us, 28672 x 4096 in two 27.9 us, 4096 x 14336
@@ -770,7 +776,13 @@ SmallPlan plan_small(int ntiles, int units, int np, int64_t chain_limit, const i
         const int64_t longest = ((int64_t)((ntiles + n - 1) / n) * units + c - 1) / c;
         const int piece = (int)(longest < units ? longest : units);
         const bool flush = np > 16 && (piece + chains - 1) / chains > limit;
-        const double t = (double)longest + (c == 1 ? 0.0 : c == 2 ? 1.0 : 9.0);
+        double exchange = c == 1 ? 0.0 : c == 2 ? 1.0 : 9.0;
+        if (c > 2 && ntiles <= n) {                          // a tile per cluster
+            if (units <= 16) exchange = c * n <= clusters[2] ? 0.5 * c : 9.0;
+            else if (np > 64) exchange = 4.0;
+            else if (c == 4 && c * n * 2 <= 3 * clusters[2]) exchange = 7.5;
+        }
+        const double t = (double)longest + exchange;
         if (t < t_best) { t_best = t; best.cluster = c; best.nclusters = n; best.flush = flush ? limit : 0; }
     }
     return best;

@@ -147,7 +147,7 @@ def errors(y, ref):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,ns,k", [
-    (65, (2048,), 2048), (65, (4096,), 4096), (96, (4096,), 4096), (128, (4096,), 4096), (100, (6144,), 4096),
+    (17, (3000,), 4096), (48, (2048,), 2048), (40, (4096,), 2048), (65, (2048,), 2048), (65, (4096,), 4096), (96, (4096,), 4096), (128, (4096,), 4096), (100, (6144,), 4096),
     (65, (8192,), 8192), (72, (3000,), 8192), (65, (4096,), 14336), (128, (4096,), 14336), (80, (12288,), 14336),
     (128, (12288,), 14336), (65, (8192,), 28672), (96, (8192,), 28672), (128, (8192,), 28672), (48, (12288,), 14336),
     (17, (4096, 1024, 1024), 4096), (48, (4096, 1024, 1024), 4096), (32, (8192, 1024, 1024), 8192),
