@@ -328,7 +328,8 @@ MIXFP4_API int mixfp4_check_status(const int* dev_status, int* value, void* stre
  * 128 or an x that TMA cannot address: MIXFP4_E_WORKSPACE without it) followed by room for
  * split-K partial sums (problems with few output tiles and a long K run several CTAs per tile;
  * optional: with a smaller or NULL workspace one CTA per tile does the whole K range, the result
- * then differs in fp32 summation order only) and a 256-byte slot used by mixfp4_gemm_a4.
+ * then differs in fp32 summation order only; n = 0 asks for no such room, which the kernel and stream layouts
+ * do not use up to 128 rows) and a 256-byte slot used by mixfp4_gemm_a4.
  * status: optional device int[1]; non-zero after completion if a bounded device-side
  * wait gave up (the output is then invalid). */
 MIXFP4_API int64_t mixfp4_gemm_workspace_bytes(int64_t m, int64_t n, int64_t k);

@@ -965,8 +965,8 @@ static int gemm_run(const void* x, int64_t m, int64_t ldx, const uint8_t* codes,
         xa = workspace;
     }
 
-    // a few dozen tokens: the decode of the weight is the work (gemm_small.cu; at 48 tokens 15 us against 35 for this
-    // file's tiles on a 4096 x 14336 weight, at 128 20 against 39).  The canonical layout keeps the tiles.
+    // a few dozen tokens: the decode of the weight is the work (gemm_small.cu; on a 4096 x 14336 weight 18 us at 48 tokens
+    // against 29 for this file's tiles, at 128 tokens 21 against 33).  The canonical layout keeps the tiles.
     if (layout != MIXFP4_LAYOUT_CANONICAL && m <= kSmallMaxTokens) {
         const mixfp4_gemv_segment seg = {codes, scales, global_scale, lut, y, ldy, n};
         const bool dependent = rotation_block == 128 || ((x_from_previous_kernel || overlap_previous) && xa == x);
@@ -997,8 +997,8 @@ static int gemm_run(const void* x, int64_t m, int64_t ldx, const uint8_t* codes,
     // More than 256 tokens and enough tiles to occupy most SMs: CTA pairs (two SMs share each decoded
     // weight tile; measured 1.25-1.3 x the single-CTA kernel at M >= 2048, slower below about 100 CTAs).
     // Pairs of 256-row CTAs unless pairs of 128-row CTAs pad the token rows noticeably less.  With at
-    // most 256 tokens a pair's second CTA would hold no rows and still decode: measured 88 us against 51
-    // for the single-CTA kernel at M = 17 .. 128 on a 28672 x 4096 weight.
+    // most 256 tokens a pair's second CTA would hold no rows and still decode: measured (canonical layout) 88 us
+    // against 51 for the single-CTA kernel at M = 17 .. 128 on a 28672 x 4096 weight.
     // the rotation pass above (or the caller's last kernel) is this launch's only producer
     const bool dep = rotation_block == 128 || (x_from_previous_kernel && xa == x);
     if (m > 256) {

@@ -20,6 +20,7 @@ from .quant import (HIGH_PRECISION_MODES, PackedWeight, _MODE_CODE, fake_quantiz
 
 GEMV_MAX_M = 16
 GROUPED_MAX_M = 64       # rows of x that mixfp4_gemm_grouped takes
+SMALL_MAX_M = 128        # rows that run without split-K partial sums on the kernel and stream layouts
 _workspaces: dict[tuple, torch.Tensor] = {}
 _status_words: dict[str, torch.Tensor] = {}
 
@@ -152,7 +153,8 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
                     fused = 128
                 else:
                     x2 = _rotation.apply_transform(x2, spec, rounding="once")
-            nbytes = lib.mixfp4_gemm_workspace_bytes(m, packed.n, packed.k)
+            partials = packed.layout == "canonical" or m > SMALL_MAX_M
+            nbytes = lib.mixfp4_gemm_workspace_bytes(m, packed.n if partials else 0, packed.k)
             ws = _workspace(x.device, nbytes)
             st = lib.mixfp4_gemm(x2.data_ptr(), m, x2.stride(0), packed.codes.data_ptr(), packed.scales.data_ptr(),
                                  nat.ptr(packed.fmt), packed.global_scale.data_ptr(), packed.n, packed.k,
@@ -171,7 +173,8 @@ def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dty
 
     Decode shapes (at most 16 rows of x), up to three kernel- or stream-layout weights without a folded
     rotation: one launch (``mixfp4_gemv_grouped``); 17 to 64 rows of x and stream-layout weights: one launch
-    too (``mixfp4_gemm_grouped``).  Anything else: one ``mixfp4_linear`` per weight, same results.
+    too (``mixfp4_gemm_grouped``; K is cut for all its weights together, so its fp32 sums can differ from separate
+    calls in their order).  Anything else: one ``mixfp4_linear`` per weight.
     """
     if not packs:
         return []

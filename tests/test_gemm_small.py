@@ -12,6 +12,7 @@ import torch
 
 import mixfp4_b200 as mx
 from mixfp4_b200 import _native as nat
+from mixfp4_b200 import linear
 from mixfp4_b200 import synth
 
 
@@ -192,3 +193,15 @@ def test_decode_sizes_report_to_the_decode_kernels_word(monkeypatch, m, own):
         check(y, x, wd, k, torch.float32)
     monkeypatch.undo()
     assert mx.decode_status() == 0 and mx.gemm_status() == 0
+
+
+@pytest.mark.gpu
+def test_no_workspace_is_kept_for_partial_sums_that_nothing_writes():
+    m, n, k = 128, 4096, 14336
+    packed = gpu_weight(n, k, 1).to_stream_layout()
+    x = synth.activations(m, k, m).cuda()
+    linear._workspaces.clear()
+    y = mx.mixfp4_linear(x, packed)
+    assert sum(w.numel() for w in linear._workspaces.values()) <= m * k * 2 + 4096
+    mx.mixfp4_linear(x, packed.to_canonical())                       # the tiles: room for their partial sums
+    assert torch.equal(mx.mixfp4_linear(x, packed), y)
