@@ -851,6 +851,31 @@ def run_kernel(args):
         print(json.dumps({"kernel": "gemm", "layout": args.layout, "n": n, "k": k, "m": m, "h128": bool(args.rotate),
                           "us": round(t * 1e6, 1), "tflops": round(2.0 * m * n * k / t / 1e12, 1),
                           "us_eager_calls": round(t_eager * 1e6, 1), "gemm_status": mx.gemm_status()}))
+    elif args.kernel == "convert":
+        layers = [torch.nn.Linear(k, n, bias=False, device="meta") for _ in range(max(2, int(400e6 // (2 * n * k))))]
+        for i, layer in enumerate(layers):
+            layer.weight = torch.nn.Parameter(weight(i), requires_grad=False)
+        state = {"i": 0}
+
+        def run():
+            state["i"] = (state["i"] + 1) % len(layers)
+            mx.MixFP4Linear.from_linear(layers[state["i"]], rotation="H128" if args.rotate else None)
+
+        t = timed(run, args.steps)
+        algo = 2 * n * k + mx.packed_nbytes(n, k)
+        print(json.dumps({"kernel": "convert", "n": n, "k": k, "h128": bool(args.rotate), "us": round(t * 1e6, 1),
+                          "gbs": round(algo / t / 1e9, 1)}))
+    elif args.kernel == "fake":
+        xs = [weight(i).float() for i in range(max(2, int(400e6 // (4 * n * k))))]
+        state = {"i": 0}
+
+        def run():
+            state["i"] = (state["i"] + 1) % len(xs)
+            mx.quant_mixfp4_granularity(xs[state["i"]], format_region="n8k64")
+
+        t = timed(run, args.steps)
+        print(json.dumps({"kernel": "fake", "n": n, "k": k, "region": "n8k64", "dtype": "f32", "us": round(t * 1e6, 1),
+                          "gbs": round(8 * n * k / t / 1e9, 1)}))
     else:
         ws = [weight(i) for i in range(max(2, int(400e6 // (2 * n * k))))]
         state = {"i": 0}
@@ -877,11 +902,11 @@ def main():
                     help="multi-GPU: GEMV + NCCL all-reduce instead of the fused GEMV + all-reduce kernel")
     ap.add_argument("--layout", default="stream", choices=["stream", "kernel"],
                     help="packed layout of the weights the linears read (stream: 1152-byte chunks; kernel: row-major)")
-    ap.add_argument("--kernel", default=None, choices=["gemv", "gemm", "quantize"],
+    ap.add_argument("--kernel", default=None, choices=["gemv", "gemm", "quantize", "convert", "fake"],
                     help="time one kernel alone on --shape N K M instead of the decode workload")
     ap.add_argument("--shape", type=int, nargs=3, default=[14336, 4096, 1], metavar=("N", "K", "M"))
     ap.add_argument("--buffers", type=int, default=None, help="--kernel gemv: distinct weights to cycle over")
-    ap.add_argument("--rotate", action="store_true", help="--kernel gemm: H128 rotation of x inside the call")
+    ap.add_argument("--rotate", action="store_true", help="--kernel gemm: H128 rotation of x inside the call; convert: of the weight")
     args = ap.parse_args()
     if args.kernel:
         run_kernel(args)

@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         // -------------------------------------------------- weight transcoders / epilogue
         // A thread decodes a whole row of a K step.  256-row tiles: all eight warps work on every step.  128-row tiles:
         // two groups of four warps take the steps in turn, so that the waits, look-ups and fences of one step run under
-        // the other group's decode (14336 x 4096 at 256 tokens 44.0 -> 39.0 us, 4096 x 4096 at 512 32.9 -> 28.8 us).
+        // the other group's decode (4096 x 4096 at 512 tokens 31.3 -> 27.1 us, 14336 x 4096 at 256 tokens 37.1 -> 36.4 us).
         constexpr int kGroups = C::kGroups;
         static_assert(kStages % kGroups == 0 && (kWStages % kGroups == 0), "a stage belongs to one transcoder group");
         const int grp = kGroups == 2 ? (warp - 2) >> 2 : 0;
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
         // -------------------------------------------------- weight transcoders / epilogue
         // Two groups of four warps take the K steps in turn, a thread a whole row of the half tile: the waits, table
         // look-ups and fences of one step run under the other group's decode (all eight warps on every step: 4096 x 14336
-        // at 777 tokens 121 us, so 89; 28672 x 8192 at 4096 tokens 1490 and 1471).
+        // at 777 tokens 117 us, so 86; 28672 x 8192 at 4096 tokens equal within the repeats, 1.46 to 1.49 ms).
         static_assert(kStages % 2 == 0 && kWStages % 2 == 0, "a stage belongs to one transcoder group");
         const int grp = (warp - 2) >> 2, row = ((warp - 2) & 3) * 32 + lane;
         const uint32_t last_row = (uint32_t)a.n - 1;

@@ -766,9 +766,9 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
 //   clusters of four on three quarters of the SMs (3000 x 4096, 17 tokens: 12.6 and 9.6 us alone, 8.4 and 8.1 us in a chain).
 // With nine there these took longer alone than the 128-row tiles (9.8 us for the first, 11.0 us for the last).
 // One decode step of 48 tokens through the linears of eight 8B-shaped decoder layers: 1358 us with the 128-row tiles of
-// gemm_kernel (seven launches and up to seven split-K sums a layer), 508 us with four launches of this kernel.  Launches
-// alone, 48 tokens: 4096 x 4096 8.7 us, 6144 x 4096 in three weights 10.6 us, 28672 x 4096 in two 27.9 us, 4096 x 14336
-// 17.3 us.  The decode's byte permutes keep the ALU busy for 476 cycles of a unit.
+// gemm_kernel (seven launches and up to seven split-K sums a layer), 514 us with four launches of this kernel.  Launches
+// in a chain, 48 tokens: 4096 x 4096 8.9 us, 6144 x 4096 in three weights 10.3 us, 28672 x 4096 in two 26.6 us, 4096 x 14336
+// 16.9 us.  The decode's byte permutes keep the ALU busy for 476 cycles of a unit.
 //
 // chain_limit (products, a multiple of 128): a chain of the tensor core's accumulation is no longer than that.  The longest
 // piece of a run is cut by the accumulators it has in turn; where that is not enough its accumulators are flushed
