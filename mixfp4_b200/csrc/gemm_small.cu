@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
         const uint32_t lut_lane = base + L.lut + (lane & ((1 << a.lut_shift) - 1)) * 16;
         const uint32_t row_lane = (uint32_t)(q * 32) << 16;
         bool ok = true;
-        const int w_shift = 31 - __clz(a.w_stages);
+        const int w_shift = 31 - __clz(a.w_stages), u_held = g < a.a_stages ? g + kGroups : g;   // first unit whose stage x can hold up
         int tile = t0 + tile_first, sub = sub_first + g;            // of this group's unit
         // kernel layout: the row's eight scale bytes of a unit, fetched while the group's unit before is decoded
         auto fetch_scales = [&](int t, int u_k) {
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) gemm_small_kernel(const __grid_c
                     for (int j = 0; j < 4; ++j) { out[8 * b + j] = p0[j]; out[8 * b + 4 + j] = p1[j]; }
                 }
                 if (h == 0) {
-                    if (u >= a.a_stages && u < a.a_stages + kGroups) wait_previous_grid();
+                    if (u == u_held) wait_previous_grid();
                     ok = wait_stage(u);
                     if (!ok) break;
                     tcgen05_fence_after();                          // the MMAs that read this stage are done
@@ -766,8 +766,8 @@ int max_clusters(int (&out)[kMaxCluster + 1]) {
 //   clusters of four on three quarters of the SMs (3000 x 4096, 17 tokens: 12.6 and 9.6 us alone, 8.4 and 8.1 us in a chain).
 // With nine there these took longer alone than the 128-row tiles (9.8 us for the first, 11.0 us for the last).
 // One decode step of 48 tokens through the linears of eight 8B-shaped decoder layers: 1358 us with the 128-row tiles of
-// gemm_kernel (seven launches and up to seven split-K sums a layer), 514 us with four launches of this kernel.  Launches
-// in a chain, 48 tokens: 4096 x 4096 8.9 us, 6144 x 4096 in three weights 10.3 us, 28672 x 4096 in two 26.6 us, 4096 x 14336
+// gemm_kernel (seven launches and up to seven split-K sums a layer), 511 us with four launches of this kernel.  Launches
+// in a chain, 48 tokens: 4096 x 4096 8.9 us, 6144 x 4096 in three weights 10.3 us, 28672 x 4096 in two 26.3 us, 4096 x 14336
 // 16.9 us.  The decode's byte permutes keep the ALU busy for 476 cycles of a unit.
 //
 // chain_limit (products, a multiple of 128): a chain of the tensor core's accumulation is no longer than that.  The longest

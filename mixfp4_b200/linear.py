@@ -87,17 +87,18 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
     nat.require_cuda(x, "x")
     if x.dtype != torch.bfloat16:
         raise TypeError("x must be bfloat16")
-    if x.shape[-1] != packed.k:
-        raise ValueError(f"x has K={x.shape[-1]}, the packed weight K={packed.k}")
+    shape, k = x.shape, packed.k
+    if shape[-1] != k:
+        raise ValueError(f"x has K={shape[-1]}, the packed weight K={k}")
     out_dtype = x.dtype if out_dtype is None else out_dtype
     if out_dtype not in (torch.float32, torch.bfloat16):
         raise TypeError("out_dtype must be float32 or bfloat16")
-    lead = x.shape[:-1]
+    lead = shape[:-1]
     # a view only where it changes something: more dimensions, or a single row, whose stride can be any number
-    x2 = x if x.dim() == 2 and (x.shape[0] > 1 or x.stride(0) == packed.k) else x.reshape(-1, packed.k)
+    x2 = x if len(shape) == 2 and (shape[0] > 1 or x.stride(0) == k) else x.reshape(-1, k)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
-    m = x2.shape[0]
+    m = shape[0] if len(shape) == 2 else x2.shape[0]
     spec = None
     if rotate is None:
         rotate = packed.rotation is not None
@@ -164,7 +165,7 @@ def mixfp4_linear(x: torch.Tensor, packed: PackedWeight, *, bias: torch.Tensor |
             nat.check("mixfp4_gemm", st)
     if bias is not None:
         y += bias.to(y.dtype)
-    return y if x.dim() == 2 else y.reshape(*lead, packed.n)
+    return y if len(shape) == 2 else y.reshape(*lead, packed.n)
 
 
 def mixfp4_linear_grouped(x: torch.Tensor, packs: list[PackedWeight], *, out_dtype: torch.dtype | None = None,
