@@ -934,6 +934,7 @@ extern "C" int mixfp4_gemm_grouped(const void* x, int64_t m, int64_t ldx, int64_
         if (in.n <= 0 || in.n > 0x7fffffffLL || in.ldy < in.n) return MIXFP4_E_SHAPE;
         if (!aligned(in.codes, 16) || (in.lut && !aligned(in.lut, 16))) return MIXFP4_E_ALIGN;
     }
+    if (!aligned(x, 16) || ldx % 8 != 0) return MIXFP4_E_ALIGN;
     const bool decode = m <= 16;                       // rows that the decode kernels take: their wait limit, their status word
     if (decode && !status) {
         if (const int rc = stream_status_word(&status)) return rc;

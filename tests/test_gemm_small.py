@@ -125,6 +125,7 @@ def test_grouped_entry_checks_its_arguments():
     assert call(m=0) == nat.E_SHAPE and call(m=65) == nat.E_SHAPE and call(count=4) == nat.E_SHAPE and call(ldx=63) == nat.E_SHAPE
     assert call(out=nat.F16) == nat.E_DTYPE
     assert call(x=ctypes.c_void_p(8)) == nat.E_ALIGN and call(ldx=68) == nat.E_ALIGN
+    assert call(m=9, x=ctypes.c_void_p(8)) == nat.E_ALIGN and call(m=9, ldx=68) == nat.E_ALIGN
     seg[0].ldy = 63
     assert call() == nat.E_SHAPE
     seg[0].ldy, seg[0].codes = 64, 8
